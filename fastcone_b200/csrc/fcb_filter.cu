@@ -4,9 +4,13 @@
 // (fastcone.py:260-292): cosine weight, zero-padding to 2W with the data at [0, W), real
 // FFT, multiplication by pi*|fftfreq(2W)| (DC bin = 1/8 of the first bin), inverse FFT,
 // crop to [0, W).  The apodised variants cosrampfilter / gaussrampfilter (fastcone.py:
-// 294-319) transform rows of length W unpadded.  The FFTs are cuFFT batched R2C/C2R
-// transforms over row batches; the weighting, padding, filter multiply, crop, 1/L scaling
-// and the cast to the storage type are this file's kernels.
+// 294-319) transform rows of length W unpadded.
+//
+// All of these are convolutions of a row with a fixed even kernel of W lags, so rows up to
+// rf::RC_MAX_W values run in one kernel that reads and writes each projection once
+// (fcb_rowfft.cuh; the bound there is instruction issue and shared memory, not HBM).  Longer
+// rows keep cuFFT's batched R2C / C2R transforms with this file's pad / multiply / crop passes:
+// 64 x 256 rows of 4500 take 2.0 ms there, of 4096 0.41 ms in the one kernel (1.4 ms before).
 #include <cufft.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -16,10 +20,100 @@
 #include <vector>
 
 #include "fcb_internal.h"
+#include "fcb_rowfft.cuh"
 
 namespace fcb {
 
-// The three element-wise passes run on 2-D grids: x over a row's elements, y over the
+// Rows of the FDK filter for rf::rowconv_kernel: cosine weight on the way in, the cast to the
+// storage type on the way out.
+struct FdkRows {
+  const float* in;
+  void* out;
+  const float* zorig;
+  float D;
+  int outType, H, W, pitch, cosw;
+  int vin, vout;  // pairs of values can be read / written as one word
+  struct Row {
+    float d, q0, c2;  // weight of column ww: d / sqrt(q0 + c2 ww^2)
+  };
+  __device__ __forceinline__ Row row(long long gr) const
+  {
+    Row r{D, 1.0f, 1.0f};
+    if (cosw) {
+      const long long t = gr >> 31 ? gr / H : (long long)((unsigned)gr / (unsigned)H);
+      const float hh = (float)(gr - t * H) - __ldg(zorig + t);
+      r.q0 = fmaxf(D * D + hh * hh, 1e-36f);
+      // where ww^2 is lost in q0 (or q0 overflows) the row has one weight
+      if (r.q0 > 1e30f) r = Row{D / sqrtf(r.q0), 1.0f, 0.0f};
+      else if (isnan(hh)) r.q0 = hh;
+    }
+    return r;
+  }
+  // D / sqrt(D^2 + hh^2 + ww^2): one Newton step brings the approximate reciprocal square
+  // root to the error of a correctly rounded root and division, at a fifth of their instructions
+  __device__ __forceinline__ float weight(const Row& r, int i) const
+  {
+    const float ww = (float)i - 0.5f * (float)W;
+    const float q = fmaf(r.c2 * ww, ww, r.q0);
+    const float s = rsqrtf(q);
+    return r.d * fmaf(0.5f * s, fmaf(-q * s, s, 1.0f), s);
+  }
+  __device__ __forceinline__ rf::cf load(long long gr, int n) const
+  {
+    const int i = 2 * n;
+    rf::cf v = {0.0f, 0.0f};
+    if (i >= W) return v;
+    const float* p = in + gr * pitch + i;
+    if (vin && i + 1 < W) {
+      const float2 t = *reinterpret_cast<const float2*>(p);
+      v = {t.x, t.y};
+    } else {
+      v.x = p[0];
+      if (i + 1 < W) v.y = p[1];
+    }
+    return v;
+  }
+  __device__ __forceinline__ rf::cf weigh(const Row& r, int n, rf::cf v) const
+  {
+    if (cosw) {  // (values beyond the row are zero and stay zero)
+      v.x *= weight(r, 2 * n);
+      v.y *= weight(r, 2 * n + 1);
+    }
+    return v;
+  }
+  __device__ __forceinline__ void store(long long gr, int n, rf::cf v) const
+  {
+    const int i = 2 * n;
+    if (i >= W) return;
+    const long long o = gr * pitch + i;
+    const bool both = i + 1 < W;
+    if (outType == FCB_F32) {
+      float* p = reinterpret_cast<float*>(out) + o;
+      if (vout && both) *reinterpret_cast<float2*>(p) = make_float2(v.x, v.y);
+      else {
+        p[0] = v.x;
+        if (both) p[1] = v.y;
+      }
+    } else {
+      unsigned short lo, hi;
+      if (outType == FCB_F16) {
+        lo = __half_as_ushort(__float2half_rn(v.x));
+        hi = __half_as_ushort(__float2half_rn(v.y));
+      } else {
+        lo = __bfloat16_as_ushort(__float2bfloat16_rn(v.x));
+        hi = __bfloat16_as_ushort(__float2bfloat16_rn(v.y));
+      }
+      unsigned short* p = reinterpret_cast<unsigned short*>(out) + o;
+      if (vout && both) *reinterpret_cast<unsigned*>(p) = (unsigned)lo | ((unsigned)hi << 16);
+      else {
+        p[0] = lo;
+        if (both) p[1] = hi;
+      }
+    }
+  }
+};
+
+// Rows longer than rf::RC_MAX_W: the three element-wise passes run on 2-D grids: x over a row's elements, y over the
 // batch's rows (at most 65535), so no thread divides its index.  (Measured against the
 // earlier one-dimensional form, which divided a 64-bit index per element: the same 2-4 TB/s;
 // these passes are a third of the filter's time, cuFFT the rest.)
@@ -121,10 +215,12 @@ __global__ void phantom_kernel(const __grid_constant__ PhParams P, int e0)
 
 using namespace fcb;
 
-// Reusable filter: cuFFT plans, scratch (padded rows, spectra) and the filter response made
-// once; execute() is stream-ordered, allocates nothing and does not synchronise.
+// Reusable filter: the row transform's tables (long rows: cuFFT plans, padded rows, spectra and
+// the filter response) made once; execute() is stream-ordered, allocates nothing and does not
+// synchronise.
 struct fcb_filter_plan {
   int nviews = 0, H = 0, W = 0, outType = FCB_F32, window = FCB_FILTER_RAMLAK;
+  rf::RowConv conv;  // rows up to rf::RC_MAX_W; the members below serve longer ones
   int n2 = 0, nb = 0, batch = 0;
   float* pad = nullptr;
   cufftComplex* spec = nullptr;
@@ -150,7 +246,7 @@ struct fcb_filter_plan {
 //  GAUSSRAMP (fastcone.gaussrampfilter, fastcone.py:306-319): L = W, a_k times a Gaussian of
 //    standard deviation gaussScale * W centred at (W - 1) / 2 and shifted by -W/2 samples
 //    (zero beyond the last sample), i.e. exp(-((k + 1/2) / sigma)^2 / 2) for k + W/2 <= W - 1.
-static int filter_response(int W, int window, double gaussScale, int* L, std::vector<float>& filt)
+static int filter_response(int W, int window, double gaussScale, int* L, std::vector<double>& filt)
 {
   if (window == FCB_FILTER_RAMLAK || window == FCB_FILTER_SHEPPLOGAN) {
     *L = 2 * W;
@@ -162,7 +258,7 @@ static int filter_response(int W, int window, double gaussScale, int* L, std::ve
     return set_error(FCB_ERR_INVALID, "unknown filter window");
   }
   const int nb = *L / 2 + 1;
-  filt.assign(nb, 0.0f);
+  filt.assign(nb, 0.0);
   for (int k = 0; k < nb; k++) {
     double f;
     if (*L == 2 * W) {
@@ -184,7 +280,7 @@ static int filter_response(int W, int window, double gaussScale, int* L, std::ve
         f = src <= (double)(W - 1) ? a * exp(-0.5 * d * d) : 0.0;
       }
     }
-    filt[k] = (float)f;
+    filt[k] = f;
   }
   return FCB_OK;
 }
@@ -197,13 +293,27 @@ try {
   if (nviews <= 0 || H <= 0 || W <= 0) return set_error(FCB_ERR_INVALID, "bad filter sizes");
   if (outType != FCB_F32 && outType != FCB_F16 && outType != FCB_BF16)
     return set_error(FCB_ERR_INVALID, "unknown output type");
-  std::vector<float> filt;
+  std::vector<double> filt;
   int L = 0;
   FCB_TRY(filter_response(W, window, gaussScale, &L, filt));
   auto* pl = new fcb_filter_plan();
   pl->nviews = nviews; pl->H = H; pl->W = W; pl->outType = outType; pl->window = window;
   pl->n2 = L;
   pl->nb = L / 2 + 1;
+  if (W <= rf::RC_MAX_W) {
+    int rc = pl->conv.create(W, filt.data(), pl->nb, L);
+    if (rc == FCB_OK && cudaMalloc(&pl->dz, nviews * sizeof(float)) != cudaSuccess) {
+      cudaGetLastError();
+      rc = set_error(FCB_ERR_NOMEM, "filter scratch");
+    }
+    if (rc) {
+      delete pl;
+      return rc;
+    }
+    *out = pl;
+    return ok();
+  }
+  const std::vector<float> filt32(filt.begin(), filt.end());
   const long long rows = (long long)nviews * H;
   // rows per cuFFT batch: about 256 MB of padded rows, at most 65535 (the kernels' grid y)
   pl->batch = (int)std::min<long long>(std::min<long long>(rows, 65535),
@@ -218,7 +328,7 @@ try {
       rc = set_error(FCB_ERR_NOMEM, "filter scratch");
       break;
     }
-    if (cudaMemcpy(pl->dfilt, filt.data(), pl->nb * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (cudaMemcpy(pl->dfilt, filt32.data(), pl->nb * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) {
       rc = set_error(FCB_ERR_CUDA, "filter response upload failed");
       break;
     }
@@ -259,6 +369,13 @@ int filter_plan_run(fcb_filter_plan* pl, const float* in, void* out, int nviews,
   if (cosineWeight && (!dzorig || !(D > 0.0f)))
     return set_error(FCB_ERR_INVALID, "cosine weighting needs D > 0 and zOrigin");
   const int n2 = pl->n2, nb = pl->nb, W = pl->W, H = pl->H, batch = pl->batch;
+  if (W <= rf::RC_MAX_W) {
+    const int es = dtype_size(pl->outType);
+    FdkRows io{in, out, dzorig, D, pl->outType, H, W, pitch, cosineWeight ? 1 : 0, 0, 0};
+    io.vin = pitch % 2 == 0 && (uintptr_t)in % 8 == 0;
+    io.vout = pitch % 2 == 0 && (uintptr_t)out % (2 * es) == 0;
+    return pl->conv.run<false>(io, (long long)nviews * H, st);
+  }
   if (cufftSetStream(pl->pf, st) != CUFFT_SUCCESS || cufftSetStream(pl->pi, st) != CUFFT_SUCCESS)
     return set_error(FCB_ERR_CUDA, "cufftSetStream failed");
   const float scale = 1.0f / (float)n2;
