@@ -9,25 +9,34 @@
 // direction of travel, u = s_u * w with s_u = -1 for a right-handed helix (angles and
 // height increasing together).  Stages:
 //   1. derivative at fixed ray direction  g1 = dg/dlam + (u^2+D^2)/D dg/du + u v/D dg/dv
-//      and length correction g2 = D / sqrt(u^2+D^2+v^2) g1      (deriv_kernel)
+//      and length correction g2 = D / sqrt(u^2+D^2+v^2) g1
 //   2. forward height rebinning onto kappa-lines v_k(u, psi) = P/(2 pi)(psi + psi/tan(psi) u/D)
-//      (rebin_fwd_kernel, per-(kappa, column) interpolation table built on the host in FP64)
+//      (per-(kappa, column) interpolation table built on the host in FP64); both stages are
+//      kats_kappa_kernel, which keeps g2 in shared memory
 //   3. Hilbert transform along u, band-limited kernel (1 - cos(pi n))/(pi n): a linear
-//      convolution done with cuFFT (kernel spectrum in FP64 on the host); kats_hilbert_kernel
-//      is the direct O(W^2) form, kept for comparison
-//   4. backward rebinning through the kappa-line of smallest |psi| (rebin_bwd_kernel,
+//      convolution, in place by the one-pass row transform (fcb_rowfft.cuh), for rows above
+//      rf::RC_MAX_W by cuFFT on zero-padded rows; kats_hilbert_kernel is the direct O(W^2) form,
+//      kept for comparison
+//   4. backward rebinning through the kappa-line of smallest |psi| (kats_rebin_bwd_kernel,
 //      per-(row, column) table).
+// The views go through in batches.  On the 736 x 64 helix of 4640 views (one B200) the filter
+// takes 3.5 ms: 2.1 ms row transforms of 594,000 kappa rows (issue-bound, see there), 1.0 ms
+// kappa rows (issue 60 %, the L2 latency of tables and views), 0.4 ms backward rebinning; with
+// whole-array passes and cuFFT it took 9.0 ms, with the forward rebinning inside the row
+// transform's loads 6.1 ms (each warp's dependent table-then-tap loads stalled the transform).
 // Backprojection with weight U over each voxel's PI interval and norm dlam/(2 pi D) then
 // reconstructs (fdk_tma_kernel with the Tam-Danielsson window).
 #include <cufft.h>
 #include <math.h>
 #include <stdint.h>
 #include <stdlib.h>
+#include <string.h>
 
 #include <algorithm>
 #include <vector>
 
 #include "fcb_internal.h"
+#include "fcb_rowfft.cuh"
 
 namespace fcb {
 
@@ -70,109 +79,114 @@ struct KatsDerivConst {
   float pw, D, iD, su;
 };
 
-template <int CPT>
-__global__ void kats_deriv_kernel(const float* __restrict__ g, float* __restrict__ g2, int n, int H,
-                                  int W, const KatsDerivConst K)
+// One column of one view: where the differences read (central inside, one-sided at the ends:
+// numpy.gradient, edge order 1) and their step sizes.
+struct KatsColumn {
+  const float *m, *c, *p;  // views t - 1, t, t + 1; the view itself beyond the ends
+  int i, dl, dr;           // the column, the offsets of the columns to the left and right
+  float sl, su;            // 1 / step between views and between columns
+  float q2, q2d, u;        // u^2 + D^2, the same / D, u
+};
+__device__ __forceinline__ KatsColumn kats_column(const float* m, const float* c, const float* p, int i, int W,
+                                                  const KatsDerivConst& K)
 {
-  const int Wq = W / CPT;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= H * Wq) return;
-  const int t = blockIdx.y;
-  const int j = q / Wq, i0 = (q - j * Wq) * CPT;
-  const size_t plane = (size_t)H * W;
-  const size_t o = (size_t)t * plane + (size_t)j * W + i0;
-  float c[CPT], a[CPT], b[CPT], dl[CPT], dgu[CPT], dgv[CPT], r[CPT];
-  ldv<CPT>(g + o, c);
-  // dg/dlam: central inside, one-sided at the ends (numpy.gradient, edge order 1)
-  if (n == 1) {
-#pragma unroll
-    for (int k = 0; k < CPT; k++) dl[k] = 0.0f;
-  } else if (t == 0) {
-    ldv<CPT>(g + o + plane, a);
-#pragma unroll
-    for (int k = 0; k < CPT; k++) dl[k] = (a[k] - c[k]) * K.idl;
-  } else if (t == n - 1) {
-    ldv<CPT>(g + o - plane, b);
-#pragma unroll
-    for (int k = 0; k < CPT; k++) dl[k] = (c[k] - b[k]) * K.idl;
-  } else {
-    ldv<CPT>(g + o + plane, a);
-    ldv<CPT>(g + o - plane, b);
-#pragma unroll
-    for (int k = 0; k < CPT; k++) dl[k] = (a[k] - b[k]) * K.hidl;
-  }
-  // dg/du with u_i = su * (i - W/2) pw; e = the row from column i0 - 1 to i0 + CPT
-  float e[CPT + 2];
-  e[0] = i0 > 0 ? g[o - 1] : 0.0f;
-#pragma unroll
-  for (int k = 0; k < CPT; k++) e[k + 1] = c[k];
-  e[CPT + 1] = i0 + CPT < W ? g[o + CPT] : 0.0f;
-#pragma unroll
-  for (int k = 0; k < CPT; k++) {
-    const int i = i0 + k;
-    if (W == 1) dgu[k] = 0.0f;
-    else if (i == 0) dgu[k] = (e[k + 2] - e[k + 1]) * K.idu;
-    else if (i == W - 1) dgu[k] = (e[k + 1] - e[k]) * K.idu;
-    else dgu[k] = (e[k + 2] - e[k]) * K.hidu;
-  }
-  if (H == 1) {
-#pragma unroll
-    for (int k = 0; k < CPT; k++) dgv[k] = 0.0f;
-  } else if (j == 0) {
-    ldv<CPT>(g + o + W, a);
-#pragma unroll
-    for (int k = 0; k < CPT; k++) dgv[k] = (a[k] - c[k]) * K.ipw;
-  } else if (j == H - 1) {
-    ldv<CPT>(g + o - W, b);
-#pragma unroll
-    for (int k = 0; k < CPT; k++) dgv[k] = (c[k] - b[k]) * K.ipw;
-  } else {
-    ldv<CPT>(g + o + W, a);
-    ldv<CPT>(g + o - W, b);
-#pragma unroll
-    for (int k = 0; k < CPT; k++) dgv[k] = (a[k] - b[k]) * K.hipw;
-  }
+  KatsColumn X;
+  X.c = c;
+  X.m = m ? m : c;
+  X.p = p ? p : c;
+  X.i = i;
+  X.sl = m && p ? K.hidl : K.idl;
+  X.dl = i > 0 ? -1 : 0;
+  X.dr = i < W - 1 ? 1 : 0;
+  X.su = X.dr - X.dl == 2 ? K.hidu : K.idu;
+  X.u = K.su * (float)(i - W / 2) * K.pw;
+  X.q2 = X.u * X.u + K.D * K.D;
+  X.q2d = X.q2 * K.iD;
+  return X;
+}
+// The derivative at fixed ray direction and the length correction at row j.  (32-bit indices
+// from the views' uniform base addresses.)
+__device__ __forceinline__ float kats_deriv(const KatsColumn& X, int j, int H, int W, const KatsDerivConst& K)
+{
+  const unsigned o = (unsigned)(j * W + X.i);
+  const unsigned up = j > 0 ? o - W : o, dn = j < H - 1 ? o + W : o;
+  const float dl = (X.p[o] - X.m[o]) * X.sl;
+  const float dgu = (X.c[o + X.dr] - X.c[o + X.dl]) * X.su;
+  const float dgv = (X.c[dn] - X.c[up]) * (j > 0 && j < H - 1 ? K.hipw : K.ipw);
   const float v = (float)(j - H / 2) * K.pw;
-#pragma unroll
-  for (int k = 0; k < CPT; k++) {
-    const float u = K.su * (float)(i0 + k - W / 2) * K.pw;
-    const float q2 = u * u + K.D * K.D;
-    const float g1 = dl[k] + (q2 * K.iD) * dgu[k] + (u * v * K.iD) * dgv[k];
-    r[k] = g1 * (K.D * rsqrtf(q2 + v * v));
-  }
-  stv<CPT>(g2 + o, r);
+  const float g1 = dl + X.q2d * dgu + (X.u * v * K.iD) * dgv;
+  return g1 * (K.D * rsqrtf(X.q2 + v * v));
 }
 
-// g3[t][k][i] = g2[t][j0][i] * (1-a) + g2[t][j0+1][i] * a from the (kappa, column) table,
-// into rows of length L whose columns [W, L) stay zero (the Hilbert transform's padding,
-// written once when the plan is made).
-template <int CPT>
-__global__ void kats_rebin_fwd_kernel(const float* __restrict__ g2, float* __restrict__ g3,
-                                      const int* __restrict__ j0tab, const float* __restrict__ atab,
-                                      int H, int W, int K, int L)
+// Derivative and forward rebinning: the kappa rows of views t0 + blockIdx.y * KK_VIEWS ... (nv of
+// them in all), columns blockIdx.x * 32 + lane, at a row pitch of L:
+//   out[tl][k][i] = g2[j0] * (1 - a) + g2[j0 + 1] * a from the (kappa, column) table (j0, a).
+// The strip's derivatives of one view sit in shared memory between the two (STAGE), since each is
+// read about 2 K / H times (the strip takes 128 bytes a row: up to 768 rows leave two CTAs per SM);
+// beyond that every tap is derived where it is read.
+// `before` is view t0 - 1 (null at the first view).
+constexpr int KK_VIEWS = 4;
+template <bool STAGE>
+__global__ void __launch_bounds__(256, 5) kats_kappa_kernel(const float* __restrict__ g,
+                                                            const float* __restrict__ before,
+                                                            float* __restrict__ out, const float2* __restrict__ tab,
+                                                            int n, int H, int W, int K, int L, int t0, int nv,
+                                                            const KatsDerivConst C)
 {
-  const int Wq = W / CPT;
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= K * Wq) return;
-  const int t = blockIdx.y;
-  const int k = q / Wq, i0 = (q - k * Wq) * CPT;
-  int j0[CPT];
-  float a[CPT], val[CPT];
-  ldv<CPT>(j0tab + (size_t)k * W + i0, j0);
-  ldv<CPT>(atab + (size_t)k * W + i0, a);
-  const float* base = g2 + (size_t)t * H * W + i0;
-#pragma unroll
-  for (int m = 0; m < CPT; m++) {
-    val[m] = 0.0f;
-    if (j0[m] >= 0) {
-      const float* col = base + m;
-      const float v0 = col[(size_t)j0[m] * W];
-      const float v1 = (j0[m] + 1 < H) ? col[(size_t)(j0[m] + 1) * W] : v0;
-      val[m] = fmaf(a[m], v1 - v0, v0);
+  extern __shared__ float kk_g2[];  // [H][32]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
+  const size_t plane = (size_t)H * W;
+  const int l0 = blockIdx.y * KK_VIEWS, l1 = min(nv, l0 + KK_VIEWS);
+  for (int tl = l0; tl < l1; tl++) {
+    const int t = t0 + tl;
+    const float* c = g + (size_t)t * plane;
+    const KatsColumn X =
+        kats_column(t == 0 ? nullptr : tl == 0 ? before : c - plane, c, t + 1 < n ? c + plane : nullptr, i, W, C);
+    if constexpr (STAGE) {
+      if (i < W) {
+#pragma unroll 2
+        for (int j = warp; j < H; j += 8) kk_g2[j * 32 + lane] = kats_deriv(X, j, H, W, C);
+      }
+      __syncthreads();
     }
+    if (i < W) {
+      float* row = out + (size_t)tl * K * L;
+#pragma unroll 4
+      for (int k = warp; k < K; k += 8) {
+        const float2 ja = __ldg(tab + (unsigned)(k * W + i));
+        const int j0 = __float_as_int(ja.x);
+        float val = 0.0f;
+        if (j0 >= 0) {  // (and at most H - 2)
+          const float v0 = STAGE ? kk_g2[j0 * 32 + lane] : kats_deriv(X, j0, H, W, C);
+          const float v1 = STAGE ? kk_g2[j0 * 32 + lane + 32] : kats_deriv(X, j0 + 1, H, W, C);
+          val = fmaf(ja.y, v1 - v0, v0);
+        }
+        row[(unsigned)(k * L + i)] = val;
+      }
+    }
+    if constexpr (STAGE) __syncthreads();
   }
-  stv<CPT>(g3 + ((size_t)t * K + k) * L + i0, val);
 }
+
+// kappa rows for rf::rowconv_kernel, in place at an even pitch of L
+struct KatsRows {
+  float* g;
+  int W, L;
+  struct Row {};
+  __device__ __forceinline__ Row row(long long) const { return Row{}; }
+  __device__ __forceinline__ rf::cf load(long long gr, int n) const
+  {
+    if (2 * n >= W) return rf::cf{0.0f, 0.0f};
+    const float2 v = *reinterpret_cast<const float2*>(g + (size_t)gr * L + 2 * n);
+    return rf::cf{v.x, 2 * n + 1 < W ? v.y : 0.0f};
+  }
+  __device__ __forceinline__ rf::cf weigh(const Row&, int, rf::cf v) const { return v; }
+  __device__ __forceinline__ void store(long long gr, int n, rf::cf v) const
+  {
+    if (2 * n < W) *reinterpret_cast<float2*>(g + (size_t)gr * L + 2 * n) = make_float2(v.x, v.y);
+  }
+};
 
 // Hilbert transform of each row along u: out[i] = sgn * sum_j h(i - j) in[j],
 // h(m) = 2 / (pi m) for odd m, 0 otherwise; one block per row (stride L), the row staged in
@@ -250,26 +264,39 @@ static double frac_index(const std::vector<double>& xs, double x)
   return lo + (x - xs[lo]) / (xs[hi] - xs[lo]);
 }
 
+static float int_bits(int v)
+{
+  float f;
+  memcpy(&f, &v, sizeof f);
+  return f;
+}
+
 // Reusable Katsevich filter for one helix and detector: the kappa-line tables, the Hilbert
-// kernel's spectrum, the cuFFT plans and the intermediate buffers are made once; execute()
-// is stream-ordered, allocates nothing and does not synchronise.
+// kernel's spectrum and the buffers of one batch of views are made once; execute() is
+// stream-ordered, allocates nothing and does not synchronise.
 struct fcb_katsevich_plan {
-  int nviews = 0, H = 0, W = 0, K = 0, L = 0, nb = 0;
-  int vb = 0;  // views per transform batch (the batch is vb * K kappa rows)
+  int nviews = 0, H = 0, W = 0, K = 0;
+  int vb = 0;  // views per batch
+  int L = 0;   // row pitch of g4 (and g3): W rounded up to 4 in the row transform, 2 W for cuFFT
   float dlam = 0.0f, pw = 0.0f, D = 0.0f, su = 0.0f;
-  float *g2 = nullptr, *dfa = nullptr, *dba = nullptr;
-  float* g3 = nullptr;  // kappa rows [views rounded up to whole batches][K][L]; [W, L) zero
-  float* g4 = nullptr;  // one batch of transformed rows [vb][K][L]
-  int *dfj = nullptr, *dbk = nullptr;
+  float2* dfja = nullptr;  // forward table
+  int* dbk = nullptr;      // backward table
+  float* dba = nullptr;
+  float* g4 = nullptr;     // kappa rows of one batch [vb][K][L], transformed in place
+  float* edge = nullptr;   // the view before a batch, when out is in
+  rf::RowConv conv;  // rows up to rf::RC_MAX_W
+  // longer rows: cuFFT
+  int nb = 0;
+  float* g3 = nullptr;  // kappa rows of one batch, [W, L) zero
   float* dhim = nullptr;
-  cufftComplex* hspec = nullptr;  // one batch of spectra
+  cufftComplex* hspec = nullptr;
   cufftHandle pf = 0, pi = 0;
   ~fcb_katsevich_plan()
   {
     if (pf) cufftDestroy(pf);
     if (pi) cufftDestroy(pi);
-    cudaFree(g2); cudaFree(g3); cudaFree(g4); cudaFree(dfa); cudaFree(dba); cudaFree(dfj);
-    cudaFree(dbk); cudaFree(hspec); cudaFree(dhim);
+    cudaFree(g3); cudaFree(g4); cudaFree(edge); cudaFree(dfja); cudaFree(dba); cudaFree(dbk);
+    cudaFree(hspec); cudaFree(dhim);
   }
 };
 
@@ -301,8 +328,9 @@ try {
   for (int i = 0; i < W; i++) umax = std::max(umax, fabs(u[i]));
   const double am = atan(umax / D);
   const double P = pitch;
-  std::vector<int> fj0((size_t)K * W), bk0((size_t)H * W);
-  std::vector<float> fa((size_t)K * W), ba((size_t)H * W);
+  std::vector<float2> fja((size_t)K * W);  // (j0 as bits, a)
+  std::vector<int> bk0((size_t)H * W);
+  std::vector<float> ba((size_t)H * W);
   std::vector<double> vk(K);
   for (int i = 0; i < W; i++) {
     for (int k = 0; k < K; k++) {
@@ -312,13 +340,11 @@ try {
       // forward: linear interpolation in v, zero outside the detector rows
       const double x = vk[k];
       if (x < v[0] || x > v[H - 1]) {
-        fj0[(size_t)k * W + i] = -1;
-        fa[(size_t)k * W + i] = 0.0f;
+        fja[(size_t)k * W + i] = make_float2(int_bits(-1), 0.0f);
       } else {
         const double f = frac_index(v, x);
         const int j0 = std::min((int)floor(f), H - 2);
-        fj0[(size_t)k * W + i] = j0;
-        fa[(size_t)k * W + i] = (float)(f - j0);
+        fja[(size_t)k * W + i] = make_float2(int_bits(j0), (float)(f - j0));
       }
     }
     for (int j = 0; j < H; j++) {
@@ -328,52 +354,74 @@ try {
       ba[(size_t)j * W + i] = (float)(f - k0);
     }
   }
-  // spectrum of the Hilbert kernel embedded in L = 2W: h(m) = 2/(pi m) for odd m,
-  // h(L-m) = -h(m); H[k] = -2 i sum_{m odd < W} h(m) sin(2 pi k m / L)
-  const int L = 2 * W, nb = W + 1;
-  std::vector<float> himag(nb);
-  for (int k = 0; k < nb; k++) {
-    double acc = 0.0;
-    for (int m = 1; m < W; m += 2) acc += (2.0 / (M_PI * m)) * sin(2.0 * M_PI * (double)k * m / L);
-    himag[k] = (float)(-2.0 * acc);
-  }
   auto* pl = new fcb_katsevich_plan();
-  pl->nviews = nviews; pl->H = H; pl->W = W; pl->K = K; pl->L = L; pl->nb = nb;
+  pl->nviews = nviews; pl->H = H; pl->W = W; pl->K = K;
   pl->dlam = (float)dlam; pl->pw = pw; pl->D = D; pl->su = (float)su;
-  // transform batches of whole views, up to 256 MiB of spectra each (larger batches gain
-  // nothing per transform and make the cuFFT plans and buffers slower to create); the
-  // kappa-row array is rounded up to whole batches and zeroed once (padding columns and rows
-  // are never written)
-  pl->vb = (int)std::min<long long>(nviews, std::max<long long>(1, (256ll << 20) / (8ll * nb * K)));
-  const long long rows_alloc = (long long)((nviews + pl->vb - 1) / pl->vb) * pl->vb * K;
-  const long long batch = (long long)pl->vb * K;
-  const size_t nhw = (size_t)nviews * H * W;
+  const bool fused = W <= rf::RC_MAX_W;
   int rc = FCB_OK;
   do {
-    if (cudaMalloc(&pl->g2, nhw * 4) || cudaMalloc(&pl->g3, (size_t)rows_alloc * L * 4) ||
-        cudaMalloc(&pl->g4, (size_t)batch * L * 4) ||
-        cudaMalloc(&pl->dfa, fa.size() * 4) || cudaMalloc(&pl->dba, ba.size() * 4) ||
-        cudaMalloc(&pl->dfj, fj0.size() * 4) || cudaMalloc(&pl->dbk, bk0.size() * 4) ||
-        cudaMalloc(&pl->hspec, (size_t)batch * nb * sizeof(cufftComplex)) || cudaMalloc(&pl->dhim, nb * 4)) {
+    if (cudaMalloc(&pl->dfja, fja.size() * sizeof(float2)) || cudaMalloc(&pl->dba, ba.size() * 4) ||
+        cudaMalloc(&pl->dbk, bk0.size() * 4)) {
+      cudaGetLastError();
+      rc = set_error(FCB_ERR_NOMEM, "Katsevich filter tables");
+      break;
+    }
+    if (cudaMemcpy(pl->dfja, fja.data(), fja.size() * sizeof(float2), cudaMemcpyHostToDevice) ||
+        cudaMemcpy(pl->dba, ba.data(), ba.size() * 4, cudaMemcpyHostToDevice) ||
+        cudaMemcpy(pl->dbk, bk0.data(), bk0.size() * 4, cudaMemcpyHostToDevice)) {
+      rc = set_error(FCB_ERR_CUDA, "Katsevich table upload failed");
+      break;
+    }
+    if (fused) {
+      rc = pl->conv.create(W, nullptr, 0, 0);
+      if (rc) break;
+      pl->L = (W + 3) & ~3;
+      // Kappa rows of a batch: up to 512 MB, whole waves of the row transform where they fill
+      // one.  Batches that stay in L2 do not pay: the three kernels are not bound by HBM, and
+      // each of their launches ends in a partly filled wave (the helix above: 64 MB of rows
+      // 4.10 ms, 128 MB 3.92, 256 MB 3.68, 512 MB 3.54, 1 GB 3.44).
+      long long budget = 512ll << 20;
+      if (const char* e = getenv("FCB_KATS_BATCH_MB")) budget = (long long)std::max(1, atoi(e)) << 20;
+      long long vb = std::max<long long>(1, budget / (4ll * pl->L * K));
+      const long long wave = pl->conv.wave_rows();
+      if (vb * K >= wave) vb = vb * K / wave * wave / K;
+      pl->vb = (int)std::min<long long>(nviews, std::max<long long>(1, vb));
+    } else {
+      // transform batches of whole views, up to 256 MiB of spectra each
+      pl->L = 2 * W;
+      pl->nb = W + 1;
+      pl->vb = (int)std::min<long long>(nviews, std::max<long long>(1, (256ll << 20) / (8ll * pl->nb * K)));
+    }
+    const long long rows = (long long)pl->vb * K;
+    if (cudaMalloc(&pl->edge, (size_t)H * W * 4) || cudaMalloc(&pl->g4, (size_t)rows * pl->L * 4)) {
       cudaGetLastError();
       rc = set_error(FCB_ERR_NOMEM, "Katsevich filter scratch");
       break;
     }
-    if (cudaMemset(pl->g3, 0, (size_t)rows_alloc * L * 4) != cudaSuccess) {
+    if (fused) break;
+    // spectrum of the Hilbert kernel embedded in L = 2W: h(m) = 2/(pi m) for odd m,
+    // h(L-m) = -h(m); H[k] = -2 i sum_{m odd < W} h(m) sin(2 pi k m / L)
+    const int L = pl->L, nb = pl->nb;
+    std::vector<float> himag(nb);
+    for (int k = 0; k < nb; k++) {
+      double acc = 0.0;
+      for (int m = 1; m < W; m += 2) acc += (2.0 / (M_PI * m)) * sin(2.0 * M_PI * (double)k * m / L);
+      himag[k] = (float)(-2.0 * acc);
+    }
+    if (cudaMalloc(&pl->g3, (size_t)rows * L * 4) || cudaMalloc(&pl->dhim, nb * 4) ||
+        cudaMalloc(&pl->hspec, (size_t)rows * nb * sizeof(cufftComplex))) {
+      cudaGetLastError();
+      rc = set_error(FCB_ERR_NOMEM, "Katsevich filter scratch");
+      break;
+    }
+    if (cudaMemset(pl->g3, 0, (size_t)rows * L * 4) != cudaSuccess ||
+        cudaMemcpy(pl->dhim, himag.data(), nb * 4, cudaMemcpyHostToDevice) != cudaSuccess) {
       rc = set_error(FCB_ERR_CUDA, "Katsevich scratch initialisation failed");
       break;
     }
-    if (cudaMemcpy(pl->dfa, fa.data(), fa.size() * 4, cudaMemcpyHostToDevice) ||
-        cudaMemcpy(pl->dba, ba.data(), ba.size() * 4, cudaMemcpyHostToDevice) ||
-        cudaMemcpy(pl->dfj, fj0.data(), fj0.size() * 4, cudaMemcpyHostToDevice) ||
-        cudaMemcpy(pl->dbk, bk0.data(), bk0.size() * 4, cudaMemcpyHostToDevice) ||
-        cudaMemcpy(pl->dhim, himag.data(), nb * 4, cudaMemcpyHostToDevice)) {
-      rc = set_error(FCB_ERR_CUDA, "Katsevich table upload failed");
-      break;
-    }
     int n1[1] = {L};
-    if (cufftPlanMany(&pl->pf, 1, n1, nullptr, 1, L, nullptr, 1, nb, CUFFT_R2C, (int)batch) != CUFFT_SUCCESS ||
-        cufftPlanMany(&pl->pi, 1, n1, nullptr, 1, nb, nullptr, 1, L, CUFFT_C2R, (int)batch) != CUFFT_SUCCESS) {
+    if (cufftPlanMany(&pl->pf, 1, n1, nullptr, 1, L, nullptr, 1, nb, CUFFT_R2C, (int)rows) != CUFFT_SUCCESS ||
+        cufftPlanMany(&pl->pi, 1, n1, nullptr, 1, nb, nullptr, 1, L, CUFFT_C2R, (int)rows) != CUFFT_SUCCESS) {
       rc = set_error(FCB_ERR_CUDA, "cufftPlanMany failed");
       break;
     }
@@ -392,13 +440,12 @@ extern "C" int fcb_katsevich_plan_execute(fcb_katsevich_plan* pl, const float* i
 try {
   if (!pl || !in || !out) return set_error(FCB_ERR_INVALID, "NULL plan or buffer");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const int nviews = pl->nviews, H = pl->H, W = pl->W, K = pl->K, L = pl->L, nb = pl->nb;
+  const int nviews = pl->nviews, H = pl->H, W = pl->W, K = pl->K, L = pl->L, nb = pl->nb, vb = pl->vb;
   // 16-byte vector accesses need 4 | W and 16-byte aligned caller buffers (the plan's own are)
   const bool v4 = (W % 4) == 0 && (reinterpret_cast<uintptr_t>(in) & 15) == 0 &&
                   (reinterpret_cast<uintptr_t>(out) & 15) == 0;
   const int cpt = v4 ? 4 : 1;
   const unsigned bx_hw = (unsigned)(((long long)H * (W / cpt) + 255) / 256);
-  const unsigned bx_kw = (unsigned)(((long long)K * (W / cpt) + 255) / 256);
   KatsDerivConst KC;
   {
     const double dl = pl->dlam, du = (double)pl->su * pl->pw, pw = pl->pw, D = pl->D;
@@ -413,39 +460,66 @@ try {
     KC.iD = (float)(1.0 / D);
     KC.su = pl->su;
   }
-  if (v4) {
-    kats_deriv_kernel<4><<<dim3(bx_hw, nviews), 256, 0, st>>>(in, pl->g2, nviews, H, W, KC);
-    kats_rebin_fwd_kernel<4><<<dim3(bx_kw, nviews), 256, 0, st>>>(pl->g2, pl->g3, pl->dfj, pl->dfa, H, W, K, L);
-  } else {
-    kats_deriv_kernel<1><<<dim3(bx_hw, nviews), 256, 0, st>>>(in, pl->g2, nviews, H, W, KC);
-    kats_rebin_fwd_kernel<1><<<dim3(bx_kw, nviews), 256, 0, st>>>(pl->g2, pl->g3, pl->dfj, pl->dfa, H, W, K, L);
-  }
-  auto rebin_bwd = [&](const float* rows, int t0, int nv, float scale) {
-    if (v4) kats_rebin_bwd_kernel<4><<<dim3(bx_hw, nv), 256, 0, st>>>(rows, out, pl->dbk, pl->dba, H, W, K, L, scale, t0);
-    else kats_rebin_bwd_kernel<1><<<dim3(bx_hw, nv), 256, 0, st>>>(rows, out, pl->dbk, pl->dba, H, W, K, L, scale, t0);
-  };
   // the published Hilbert transform runs along increasing u; along w it changes sign when u = -w
-  const char* direct = getenv("FCB_KATS_DIRECT_HILBERT");
-  if (direct && direct[0] == '1') {
-    kats_hilbert_kernel<<<(unsigned)((size_t)nviews * K), 256, W * sizeof(float), st>>>(pl->g3, W, L, pl->su);
-    rebin_bwd(pl->g3, 0, nviews, 1.0f);
-  } else {
-    if (cufftSetStream(pl->pf, st) != CUFFT_SUCCESS || cufftSetStream(pl->pi, st) != CUFFT_SUCCESS)
-      return set_error(FCB_ERR_CUDA, "cufftSetStream failed");
-    const float scale = pl->su / (float)L;
-    const int vb = pl->vb;
-    // per batch of whole views: R2C of the zero-padded kappa rows, multiplication by the
-    // kernel's spectrum, C2R into g4 (the padding in g3 stays zero), backward rebinning of
-    // the batch's views with the 1/L normalisation and the direction sign
-    for (int t0 = 0; t0 < nviews; t0 += vb) {
-      const int nv = std::min(vb, nviews - t0);
-      if (cufftExecR2C(pl->pf, pl->g3 + (size_t)t0 * K * L, pl->hspec) != CUFFT_SUCCESS)
-        return set_error(FCB_ERR_CUDA, "cufftExecR2C failed");
-      kats_spec_kernel<<<(unsigned)((long long)nv * K), 256, 0, st>>>(pl->hspec, pl->dhim, nb);
-      if (cufftExecC2R(pl->pi, pl->hspec, pl->g4) != CUFFT_SUCCESS) return set_error(FCB_ERR_CUDA, "cufftExecC2R failed");
-      rebin_bwd(pl->g4, t0, nv, scale);
+  const char* de = getenv("FCB_KATS_DIRECT_HILBERT");
+  const bool direct = de && de[0] == '1';  // the direct sum, for comparison
+  const bool fused = W <= rf::RC_MAX_W;
+  if (!fused && (cufftSetStream(pl->pf, st) != CUFFT_SUCCESS || cufftSetStream(pl->pi, st) != CUFFT_SUCCESS))
+    return set_error(FCB_ERR_CUDA, "cufftSetStream failed");
+  // out may be in: a batch's derivatives also read the last view of the batch before, which is
+  // kept aside before that batch is written.  Buffers that overlap in some other way go through
+  // a copy.
+  const size_t plane = (size_t)H * W, nhw = (size_t)nviews * plane;
+  const float* src = in;
+  float* copy = nullptr;
+  if (in != out && in < out + nhw && out < in + nhw) {
+    FCB_CUDA_TRY(cudaMallocAsync((void**)&copy, nhw * sizeof(float), st));
+    src = copy;
+    const cudaError_t e = cudaMemcpyAsync(copy, in, nhw * sizeof(float), cudaMemcpyDeviceToDevice, st);
+    if (e != cudaSuccess) {
+      cudaFreeAsync(copy, st);
+      return set_error(FCB_ERR_CUDA, cudaGetErrorString(e));
     }
   }
+  const size_t strip = (size_t)H * 32 * sizeof(float);  // a view's derivatives in 32 columns
+  const bool stage = strip <= 96 * 1024;
+  if (stage)
+    FCB_CUDA_TRY(cudaFuncSetAttribute(kats_kappa_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+  // one batch: kappa rows of views [t0, t0 + nv), their Hilbert transform, backward rebinning
+  auto batch = [&](int t0, int nv) -> int {
+    const long long rows = (long long)nv * K;
+    float* g3 = fused || direct ? pl->g4 : pl->g3;
+    const float* before = t0 == 0 ? nullptr : in == out ? pl->edge : src + (size_t)(t0 - 1) * plane;
+    const dim3 kg((W + 31) / 32, (nv + KK_VIEWS - 1) / KK_VIEWS);
+    if (stage) kats_kappa_kernel<true><<<kg, 256, strip, st>>>(src, before, g3, pl->dfja, nviews, H, W, K, L, t0, nv, KC);
+    else kats_kappa_kernel<false><<<kg, 256, 0, st>>>(src, before, g3, pl->dfja, nviews, H, W, K, L, t0, nv, KC);
+    FCB_CUDA_TRY(cudaGetLastError());
+    if (in == out && t0 + nv < nviews)
+      FCB_CUDA_TRY(cudaMemcpyAsync(pl->edge, in + (size_t)(t0 + nv - 1) * plane, plane * sizeof(float),
+                                   cudaMemcpyDeviceToDevice, st));
+    float scale = pl->su;
+    if (direct) {
+      kats_hilbert_kernel<<<(unsigned)rows, 256, W * sizeof(float), st>>>(g3, W, L, pl->su);
+      scale = 1.0f;
+    } else if (fused) {
+      FCB_TRY(pl->conv.run<true>(KatsRows{pl->g4, W, L}, rows, st));
+    } else {
+      // R2C of the zero-padded kappa rows (the padding in g3 stays zero), multiplication by the
+      // kernel's spectrum, C2R into g4; the backward rebinning applies 1/L and the sign
+      if (cufftExecR2C(pl->pf, g3, pl->hspec) != CUFFT_SUCCESS) return set_error(FCB_ERR_CUDA, "cufftExecR2C failed");
+      kats_spec_kernel<<<(unsigned)rows, 256, 0, st>>>(pl->hspec, pl->dhim, nb);
+      if (cufftExecC2R(pl->pi, pl->hspec, pl->g4) != CUFFT_SUCCESS) return set_error(FCB_ERR_CUDA, "cufftExecC2R failed");
+      scale = pl->su / (float)L;
+    }
+    if (v4) kats_rebin_bwd_kernel<4><<<dim3(bx_hw, nv), 256, 0, st>>>(pl->g4, out, pl->dbk, pl->dba, H, W, K, L, scale, t0);
+    else kats_rebin_bwd_kernel<1><<<dim3(bx_hw, nv), 256, 0, st>>>(pl->g4, out, pl->dbk, pl->dba, H, W, K, L, scale, t0);
+    FCB_CUDA_TRY(cudaGetLastError());
+    return FCB_OK;
+  };
+  int rc = FCB_OK;
+  for (int t0 = 0; t0 < nviews && rc == FCB_OK; t0 += vb) rc = batch(t0, std::min(vb, nviews - t0));
+  if (copy) cudaFreeAsync(copy, st);
+  if (rc) return rc;
   FCB_CUDA_TRY(cudaGetLastError());
   return ok();
 }

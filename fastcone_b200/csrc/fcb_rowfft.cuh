@@ -589,6 +589,16 @@ struct RowConv {
     FCB_CUDA_TRY(cudaStreamSynchronize(0));  // the tables are read on any stream from here on
     return FCB_OK;
   }
+  // rows that the device's row groups hold at one time
+  long long wave_rows() const
+  {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    long long n = 0;
+    rc_dispatch(W, [&](auto k) { n = (long long)decltype(k)::GPC * decltype(k)::R * sms; });
+    return n;
+  }
   // Convolves `nrows` rows through `io`, stream-ordered.
   template <bool ODD, class IO>
   int run(const IO& io, long long nrows, cudaStream_t st) const

@@ -250,8 +250,8 @@ int fcb_fdk_filter_device(const float* in, void* out, int outType, int nviews, i
                           float D, const float* zOrigin, int cosineWeight, int window,
                           void* stream);
 
-/* The same filter as a reusable plan: cuFFT plans, scratch and the filter response are made
- * once; execute is stream-ordered, allocates nothing and does not synchronise (zOrigin, host,
+/* The same filter as a reusable plan: the row transform's tables (rows above 4096 values: cuFFT
+ * plans, scratch and the filter response) are made once; execute is stream-ordered, allocates nothing and does not synchronise (zOrigin, host,
  * is read before it returns).  One execute at a time per plan (the scratch is the plan's). */
 typedef struct fcb_filter_plan fcb_filter_plan;
 int fcb_filter_plan_create(int nviews, int H, int W, int outType, int window,
@@ -277,9 +277,9 @@ int fcb_katsevich_filter_device(const float* in, float* out, int nviews, int H, 
                                 void* stream);
 
 /* The same filter as a reusable plan for one helix and detector: kappa-line tables, the
- * Hilbert kernel's spectrum, cuFFT plans and intermediate buffers made once (nviews x H x W
- * floats plus nviews x nkappa x 2W floats of zero-padded kappa rows, plus 0.5 GiB of transform
- * batches); execute is stream-ordered, allocates nothing
+ * Hilbert kernel's spectrum and the kappa rows of one batch of views made once (512 MiB at most; above
+ * 4096 columns the Hilbert transform is cuFFT's, on 0.75 GiB batches); execute is stream-ordered, allocates nothing
+ * (unless in and out overlap without being the same buffer: then a stream-ordered copy of in)
  * and does not synchronise.  One execute at a time per plan. */
 typedef struct fcb_katsevich_plan fcb_katsevich_plan;
 int fcb_katsevich_plan_create(int nviews, int H, int W, const float* angles, float D, float pw,
