@@ -92,7 +92,7 @@ bool cache_enabled()
   return !(e && e[0] == '0');
 }
 
-// fcb_fbp_host's filter plans (cuFFT plans and about half a gigabyte of scratch each) are
+// fcb_fbp_host's filter plans (the row transform's tables, or cuFFT plans and their scratch) are
 // kept the same way, keyed by their parameters, at most 4 per device.
 struct CachedFilter {
   int dev;
@@ -789,6 +789,7 @@ extern "C" int fcb_release_device_cache(void)
 try {
   std::lock_guard<std::mutex> lk(g_cache_mu);
   cache_drop_locked(-1);
+  scratch_trim();
   return ok();
 }
 FCB_CATCH_STATUS

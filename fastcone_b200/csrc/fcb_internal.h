@@ -58,6 +58,11 @@ int device_status_ptr(int** p);
 // Unique id of the calling thread's current CUDA context (a reset device gets a new one);
 // 0 when there is none or the driver cannot tell.
 unsigned long long current_context_id();
+// Stream-ordered device scratch from the library's own per-device pool (freed memory up to 1 GiB
+// stays with it; scratch_trim returns it to the driver).
+int scratch_alloc(void** p, size_t bytes, cudaStream_t st);
+void scratch_free(void* p, cudaStream_t st);
+void scratch_trim();
 // Reads and clears the status word after synchronising `stream`.
 int collect_device_status(cudaStream_t stream);
 

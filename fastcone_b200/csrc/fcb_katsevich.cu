@@ -473,11 +473,11 @@ try {
   const float* src = in;
   float* copy = nullptr;
   if (in != out && in < out + nhw && out < in + nhw) {
-    FCB_CUDA_TRY(cudaMallocAsync((void**)&copy, nhw * sizeof(float), st));
+    FCB_TRY(scratch_alloc((void**)&copy, nhw * sizeof(float), st));
     src = copy;
     const cudaError_t e = cudaMemcpyAsync(copy, in, nhw * sizeof(float), cudaMemcpyDeviceToDevice, st);
     if (e != cudaSuccess) {
-      cudaFreeAsync(copy, st);
+      scratch_free(copy, st);
       return set_error(FCB_ERR_CUDA, cudaGetErrorString(e));
     }
   }
@@ -518,7 +518,7 @@ try {
   };
   int rc = FCB_OK;
   for (int t0 = 0; t0 < nviews && rc == FCB_OK; t0 += vb) rc = batch(t0, std::min(vb, nviews - t0));
-  if (copy) cudaFreeAsync(copy, st);
+  scratch_free(copy, st);
   if (rc) return rc;
   FCB_CUDA_TRY(cudaGetLastError());
   return ok();

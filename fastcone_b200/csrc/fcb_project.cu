@@ -251,30 +251,48 @@ __device__ __forceinline__ void bundle_of(const PjView& V, int bw0, int bh0, Bun
   B.sgn = (B.xdom ? c[0] : c[1]) > 0.0f ? 1 : -1;
 }
 
-// Brick of the slab whose samples have floor(dominant) in [a, a + T - 1]: the frustum's
-// cross / z range between the dominant planes a and a + T (clipped to [lo, hi]), plus
-// the +1 trilinear neighbour; the cross origin is aligned down to 4 voxels (16-byte TMA rule).
-template <int T>
-__device__ __forceinline__ void brick_extent(const Bundle& B, int a, float lo, float hi, int& c0,
-                                             int& z0, int& needc, int& needz)
+// The bundle's corner rays as functions of the dominant coordinate.
+struct BundleLines {
+  float sD, sC, sZ;                // source: dominant, cross, z
+  float inv[4], dC[4], dZ[4];      // 1 / (dominant direction), cross and z directions
+};
+__device__ __forceinline__ BundleLines lines_of(const Bundle& B)
 {
   // (selects instead of runtime array indices keep everything in registers)
   const bool xd = B.xdom != 0;
-  const float sD = xd ? B.s[0] : B.s[1], sC = xd ? B.s[1] : B.s[0];
-  float cmin = 3.0e38f, cmax = -3.0e38f, zmin = 3.0e38f, zmax = -3.0e38f;
-  const float p0 = fmaxf((float)a, lo), p1 = fminf((float)(a + T), hi);
+  BundleLines L;
+  L.sD = xd ? B.s[0] : B.s[1];
+  L.sC = xd ? B.s[1] : B.s[0];
+  L.sZ = B.s[2];
 #pragma unroll
   for (int q = 0; q < 4; q++) {
-    const float dD = xd ? B.d[q][0] : B.d[q][1], dC = xd ? B.d[q][1] : B.d[q][0];
-    const float inv = 1.0f / dD;
-#pragma unroll
-    for (int e = 0; e < 2; e++) {
-      const float t = ((e ? p1 : p0) - sD) * inv;
-      const float c = fmaf(t, dC, sC), z = fmaf(t, B.d[q][2], B.s[2]);
-      cmin = fminf(cmin, c); cmax = fmaxf(cmax, c);
-      zmin = fminf(zmin, z); zmax = fmaxf(zmax, z);
-    }
+    L.inv[q] = 1.0f / (xd ? B.d[q][0] : B.d[q][1]);
+    L.dC[q] = xd ? B.d[q][1] : B.d[q][0];
+    L.dZ[q] = B.d[q][2];
   }
+  return L;
+}
+// Cross and z range of the corner rays at the dominant coordinate p.
+__device__ __forceinline__ float4 plane_range(const BundleLines& L, float p)
+{
+  float4 r = make_float4(3.0e38f, -3.0e38f, 3.0e38f, -3.0e38f);
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const float t = (p - L.sD) * L.inv[q];
+    const float c = fmaf(t, L.dC[q], L.sC), z = fmaf(t, L.dZ[q], L.sZ);
+    r.x = fminf(r.x, c); r.y = fmaxf(r.y, c);
+    r.z = fminf(r.z, z); r.w = fmaxf(r.w, z);
+  }
+  return r;
+}
+// Brick of the slab whose samples have floor(dominant) in [a, a + T - 1]: the frustum's
+// cross / z range between the dominant planes a and a + T (clipped to [lo, hi]), plus
+// the +1 trilinear neighbour; the cross origin is aligned down to 4 voxels (16-byte TMA rule).
+__device__ __forceinline__ void brick_extent(const BundleLines& L, float4 r0, int a, int T, float lo, float hi,
+                                             int& c0, int& z0, int& needc, int& needz)
+{
+  const float4 r1 = plane_range(L, fminf((float)(a + T), hi));
+  float cmin = fminf(r0.x, r1.x), cmax = fmaxf(r0.y, r1.y), zmin = fminf(r0.z, r1.z), zmax = fmaxf(r0.w, r1.w);
   cmin = fminf(fmaxf(cmin, -1.0e6f), 1.0e6f); cmax = fminf(fmaxf(cmax, -1.0e6f), 1.0e6f);
   zmin = fminf(fmaxf(zmin, -1.0e6f), 1.0e6f); zmax = fminf(fmaxf(zmax, -1.0e6f), 1.0e6f);
   c0 = __float2int_rd(cmin) & ~3;
@@ -282,35 +300,48 @@ __device__ __forceinline__ void brick_extent(const Bundle& B, int a, float lo, f
   needc = __float2int_rd(cmax) + 2 - c0;
   needz = __float2int_rd(zmax) + 2 - z0;
 }
-
-// Pre-pass: the largest brick over every (view, bundle, slab start) sizes the staged box.
 template <int T>
-__global__ void project_brick_extent_kernel(const __grid_constant__ PjParams P, int bx, int by,
-                                            int* out)
+__device__ __forceinline__ void brick_extent(const BundleLines& L, int a, float lo, float hi, int& c0, int& z0,
+                                             int& needc, int& needz)
 {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  brick_extent(L, plane_range(L, fmaxf((float)a, lo)), a, T, lo, hi, c0, z0, needc, needz);
+}
+
+// Pre-pass: the largest brick over every (view, bundle, slab start) sizes the staged box, for the
+// three slab depths at once (out[2 i], out[2 i + 1]: cross and z extents for depth 12, 8, 6), by
+// EXT_LANES threads per bundle.  One launch and one read-back per call (256^3, 180 views: 141 us;
+// a launch of 60 us, a clear and a read-back per depth tried before).
+constexpr int EXT_LANES = 8;
+__global__ void __launch_bounds__(256) project_brick_extent_kernel(const __grid_constant__ PjParams P, int bx, int by,
+                                                                   int* out)
+{
+  constexpr int DEPTH[3] = {12, 8, 6};
+  const long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / EXT_LANES;
   const long long total = (long long)P.nviews * bx * by;
-  int mc = 0, mz = 0;
+  int m[6] = {0, 0, 0, 0, 0, 0};
   if (i < total) {
-    const int v = (int)(i / ((long long)bx * by));
-    const int b = (int)(i % ((long long)bx * by));
+    const int v = (int)(i / (bx * by));
+    const int b = (int)(i - (long long)v * (bx * by));
     Bundle B;
     bundle_of(P.v[v], (b % bx) * PB_W, (b / bx) * PB_H, B);
+    const BundleLines L = lines_of(B);
     const int ndom = B.xdom ? P.nx : P.ny;
-    for (int a = -T; a <= ndom; a++) {
-      int c0, z0, nc, nz;
-      brick_extent<T>(B, a, -1.0f, (float)ndom, c0, z0, nc, nz);
-      mc = max(mc, nc);
-      mz = max(mz, nz);
+    for (int a = -DEPTH[0] + (int)(threadIdx.x % EXT_LANES); a <= ndom; a += EXT_LANES) {
+      const float4 r0 = plane_range(L, fmaxf((float)a, -1.0f));
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        int c0, z0, nc, nz;
+        if (a < -DEPTH[d]) continue;
+        brick_extent(L, r0, a, DEPTH[d], -1.0f, (float)ndom, c0, z0, nc, nz);
+        m[2 * d] = max(m[2 * d], nc);
+        m[2 * d + 1] = max(m[2 * d + 1], nz);
+      }
     }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    mc = max(mc, __shfl_xor_sync(0xffffffffu, mc, o));
-    mz = max(mz, __shfl_xor_sync(0xffffffffu, mz, o));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicMax(out, mc);
-    atomicMax(out + 1, mz);
+#pragma unroll
+  for (int k = 0; k < 6; k++) {
+    m[k] = __reduce_max_sync(0xffffffffu, m[k]);
+    if ((threadIdx.x & 31) == 0) atomicMax(out + k, m[k]);
   }
 }
 
@@ -531,6 +562,7 @@ __global__ void __launch_bounds__(PB_THREADS, MINB) project_brick_kernel(
     const CUtensorMap* tm = B.xdom ? &tmT : &tmV;
     dev::tma_prefetch(tm);
     const uint32_t bytes = (uint32_t)(P.BC * (T + 1) * P.BZ * 4);
+    const BundleLines L = lines_of(B);
     int issued = 0;
     bool failed = false;
     for (int k = 0; k < nsl; k++) {
@@ -541,7 +573,7 @@ __global__ void __launch_bounds__(PB_THREADS, MINB) project_brick_kernel(
       }
       const int a = B.sgn > 0 ? fmin + k * T : fmax - T + 1 - k * T;
       int c0, z0, nc, nz;
-      brick_extent<T>(B, a, -1.0f, (float)ndom, c0, z0, nc, nz);
+      brick_extent<T>(L, a, -1.0f, (float)ndom, c0, z0, nc, nz);
       origin[st] = make_int4(c0, a, z0, 0);
       dev::mbar_arrive_expect_tx(&full[st], bytes);
       dev::tma_load_3d(smem_raw + (size_t)st * P.stage_bytes, tm, &full[st], c0, a, z0);
@@ -627,7 +659,7 @@ __global__ void __launch_bounds__(256, MINB) project_adjoint_brick_kernel(const 
     const int a = B.sgn > 0 ? fmin + k * T : fmax - T + 1 - k * T;
     if (threadIdx.x == 0) {
       int c0, z0, nc, nzz;
-      brick_extent<T>(B, a, -1.0f, (float)ndom, c0, z0, nc, nzz);
+      brick_extent<T>(lines_of(B), a, -1.0f, (float)ndom, c0, z0, nc, nzz);
       org[0] = make_int4(c0, a, z0, 0);
       box[0] = box[2] = box[4] = INT_MAX;
       box[1] = box[3] = box[5] = INT_MIN;
@@ -786,9 +818,23 @@ int brick_setup(const std::vector<PjParams>& chunks, int nx, int ny, cudaStream_
 {
   bs->ok = false;
   if (nx % 4 != 0 || ny % 4 != 0 || getenv("FCB_PROJ_NOBRICK")) return FCB_OK;
-  int* scratch = nullptr;
-  FCB_TRY(device_status_ptr(&scratch));
-  int* need = scratch + 3;  // [3..4]: brick extents ([1..2] belong to the backprojector)
+  // every depth's extents by one kernel per view chunk, read back once
+  int* need = nullptr;
+  FCB_TRY(scratch_alloc((void**)&need, 6 * sizeof(int), st));
+  int ext[6] = {0, 0, 0, 0, 0, 0};
+  cudaError_t ce = cudaMemsetAsync(need, 0, sizeof ext, st);
+  for (const PjParams& P : chunks) {
+    const int bx = (P.WH0 + PB_W - 1) / PB_W, by = (P.WH1 + PB_H - 1) / PB_H;
+    const long long threads = (long long)P.nviews * bx * by * EXT_LANES;
+    if (ce == cudaSuccess) {
+      project_brick_extent_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(P, bx, by, need);
+      ce = cudaGetLastError();
+    }
+  }
+  if (ce == cudaSuccess) ce = cudaMemcpyAsync(ext, need, sizeof ext, cudaMemcpyDeviceToHost, st);
+  if (ce == cudaSuccess) ce = cudaStreamSynchronize(st);
+  scratch_free(need, st);
+  FCB_CUDA_TRY(ce);
   // Slab depth, forward: the deepest of 12, 8 and 6 dominant planes with which three CTAs of
   // two brick buffers fit in an SM's shared memory, else 6 (on the 256^3 / 360-view
   // geometry 6 planes give three CTAs instead of one: 19.9 ms per pass instead of 29.7).
@@ -800,19 +846,7 @@ int brick_setup(const std::vector<PjParams>& chunks, int nx, int ny, cudaStream_
   for (int oi = 0; oi < 3; oi++) {
     const int T = for_adjoint ? order_adj[oi] : order_fwd[oi];
     if (forced && forced != T) continue;
-    FCB_CUDA_TRY(cudaMemsetAsync(need, 0, 2 * sizeof(int), st));
-    for (const PjParams& P : chunks) {
-      const int bx = (P.WH0 + PB_W - 1) / PB_W, by = (P.WH1 + PB_H - 1) / PB_H;
-      const long long total = (long long)P.nviews * bx * by;
-      const unsigned g = (unsigned)((total + 255) / 256);
-      if (T == 12) project_brick_extent_kernel<12><<<g, 256, 0, st>>>(P, bx, by, need);
-      else if (T == 8) project_brick_extent_kernel<8><<<g, 256, 0, st>>>(P, bx, by, need);
-      else project_brick_extent_kernel<6><<<g, 256, 0, st>>>(P, bx, by, need);
-      FCB_CUDA_TRY(cudaGetLastError());
-    }
-    int h[2] = {0, 0};
-    FCB_CUDA_TRY(cudaMemcpyAsync(h, need, sizeof h, cudaMemcpyDeviceToHost, st));
-    FCB_CUDA_TRY(cudaStreamSynchronize(st));
+    const int* h = ext + (T == 12 ? 0 : T == 8 ? 2 : 4);
     const int BC = std::max(4, (h[0] + 3) & ~3), BZ = std::max(2, h[1]);
     if (BC > 128 || BZ > 64) continue;  // a wide cone: bricks would not pay
     const int box = BC * (T + 1) * BZ * 4;
@@ -1048,12 +1082,12 @@ int project_launch(const Problem& pb, int method, const float* vol, float* proj,
         tab[o] = make_int4(rw.ws[o] - pb.woff[v], rw.hs[o] - pb.hoff[v], rw.sweepStart[o],
                            rw.sweepSteps[o]);
       }
-    FCB_CUDA_TRY(cudaMallocAsync((void**)&d_win, tab.size() * sizeof(int4), st));
+    FCB_TRY(scratch_alloc((void**)&d_win, tab.size() * sizeof(int4), st));
     cudaError_t e = cudaMemcpyAsync(d_win, tab.data(), tab.size() * sizeof(int4),
                                     cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);  // the table is a local vector
     if (e != cudaSuccess) {
-      cudaFreeAsync(d_win, st);
+      scratch_free(d_win, st);
       return set_error(FCB_ERR_CUDA, cudaGetErrorString(e));
     }
   }
@@ -1115,10 +1149,10 @@ int project_launch(const Problem& pb, int method, const float* vol, float* proj,
     FCB_TRY(brick_setup(chunks, nx, ny, st, &bs, adj_vol != nullptr));
     if (bs.ok) {
       float* vt = nullptr;
-      FCB_CUDA_TRY(cudaMallocAsync((void**)&vt, (size_t)nx * ny * nz * sizeof(float), st));
+      FCB_TRY(scratch_alloc((void**)&vt, (size_t)nx * ny * nz * sizeof(float), st));
       rc = adj_vol ? brick_adjoint_launch(chunks, bs, adj_vol, vt, nx, ny, nz, st)
                    : brick_launch(chunks, bs, vol, vt, nx, ny, nz, st);
-      cudaFreeAsync(vt, st);
+      scratch_free(vt, st);
       return rc;
     }
   }
@@ -1137,7 +1171,7 @@ int project_launch(const Problem& pb, int method, const float* vol, float* proj,
     cudaDestroyTextureObject(tex);
     cudaFreeArray(arr);
   }
-  if (d_win) cudaFreeAsync(d_win, st);
+  scratch_free(d_win, st);
   return rc;
 }
 
