@@ -14,8 +14,9 @@
 //    changes, so the per-view work (U, w, weight) is amortised over NZ updates.  Per-view
 //    parameters travel in the kernel's parameter space (a constant bank).
 //  * bp_generic_kernel -- any detector orientation (misalignments) through a per-view 3x4
-//    projective matrix, bilinear gathers from global memory; also the fallback for
-//    projection buffers whose layout a TMA descriptor cannot describe.
+//    projective matrix, bilinear gathers from global memory; also for misaligned base addresses,
+//    for rows that are not whole 16-byte groups under capture, without scratch or with the PI
+//    window, and for footprints too large to stage.
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
@@ -38,6 +39,14 @@ struct FdkView {
   float wc, hc;  // local window index of the detector centre (w) / source height (h)
   float e;       // h = U (hb z + e) + hc
   float wt;      // normalisation factor of the view
+};
+
+// A view of the generic kernel: its 3x4 projective matrix and weights.
+struct __align__(16) GenView {
+  float m[12];
+  float kappa;
+  float wt;
+  float wc, hc;  // local window column of the detector centre, row of the source (PI window)
 };
 
 constexpr int FDK_MAXV = 900;      // views a launch's parameters can hold
@@ -70,6 +79,7 @@ struct FdkParams {
   unsigned long long cwait_ns;
   int stop_after;
   int pbufs;                    // 16-bit storage: tap-pair buffers (fdk_pair_kernel)
+  const GenView* gen;           // MATRIX kernels: the launch's views as the generic kernel has them
   FdkView v[FDK_MAXV];
 };
 
@@ -323,6 +333,12 @@ __device__ __forceinline__ u64 sub2(u64 a, u64 b)
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
+__device__ __forceinline__ u64 mul2(u64 a, u64 b)
+{
+  u64 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
 __device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c)
 {
   u64 r;
@@ -384,12 +400,46 @@ __device__ __forceinline__ void piw_pairs(float lo, float hi, float h0, float dh
   phi = __reduce_max_sync(0xffffffffu, b);
 }
 
+// Voxel positions of the staged kernels.  The default form keeps window-local row positions and
+// steps them along z (FdkView).  MATRIX takes them from the view's projective matrix exactly as
+// bp_generic_kernel does: it serves projections whose rows TMA cannot describe, which that kernel
+// gathered from global memory, and gives the same positions and weights bit for bit.  (In the
+// aligned geometry w and the depth do not depend on z.)
+struct MatrixColumn {
+  float fw;        // fraction along w
+  int iw;          // column in the box
+  float rs, mv, bv;  // row of voxel z: (mv z + bv) rs, in the caller's window
+  float wt;
+  bool ok;         // every tap inside the box
+};
+__device__ __forceinline__ MatrixColumn matrix_column(const GenView& V, float x, float y, float z0, int nz, int wexp,
+                                                      int4 org, int BW, int BH)
+{
+  MatrixColumn c;
+  const float bu = fmaf(V.m[0], x, fmaf(V.m[1], y, V.m[3]));
+  c.bv = fmaf(V.m[4], x, fmaf(V.m[5], y, V.m[7]));
+  const float bs = fmaf(V.m[8], x, fmaf(V.m[9], y, V.m[11]));
+  c.mv = V.m[6];
+  c.rs = 1.0f / bs;
+  const float wl = bu * c.rs;
+  const float w0 = __int_as_float(org.x), h0 = __int_as_float(org.y);
+  const float fl = floorf(wl);
+  c.fw = wl - fl;
+  c.wt = V.wt;
+  if (wexp >= 1) c.wt *= V.kappa * c.rs;
+  if (wexp >= 2) c.wt *= V.kappa * c.rs;
+  const float ha = fmaf(c.mv, z0, c.bv) * c.rs - h0, hb = fmaf(c.mv, z0 + (float)(nz - 1), c.bv) * c.rs - h0;
+  c.iw = (int)(fl - w0);
+  c.ok = fl >= w0 && c.iw <= BW - 2 && ha >= 0.0f && hb + 0.01f < (float)(BH - 1) && hb >= ha;
+  return c;
+}
+
 // Resident CTAs per SM the register allocation must allow: 3 (the default 64 KB staging
 // budget fits 3 CTAs) unless NZ = 64 needs the registers of 2.
 template <int NZ>
 constexpr int fdk_min_blocks() { return NZ >= 64 ? 2 : 3; }
 
-template <typename T, int NZ, bool PIW, bool X2, int MINB = fdk_min_blocks<NZ>()>
+template <typename T, int NZ, bool PIW, bool X2, int MINB = fdk_min_blocks<NZ>(), bool MATRIX = false>
 __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid_constant__ CUtensorMap tmap,
                                                               const __grid_constant__ FdkParams P)
 {
@@ -410,6 +460,8 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
   // them from shared memory (the views of a launch overflow the constant cache while the
   // CTAs of an SM work on different views)
   FdkView* vstage = reinterpret_cast<FdkView*>(origin + P.stages);
+  static_assert(!MATRIX || (X2 && !PIW), "matrix positions");
+  GenView* gstage = reinterpret_cast<GenView*>(vstage);  // MATRIX: the same for its views
   const uint32_t smem_base = dev::smem_u32(smem_raw);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -497,8 +549,9 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
         }
         if (nw > P.BW || nh > P.BH) dev::record_status(P.status, DEV_RANGE);
         origin[s] = make_int4(__float_as_int((float)w0), __float_as_int((float)h0), v, nh);
-        vstage[s] = P.v[v];
-        dev::mbar_arrive_expect_tx(&full[s], bytes);
+        if constexpr (!MATRIX) vstage[s] = P.v[v];
+        dev::mbar_arrive_expect_tx(&full[s], bytes + (MATRIX ? (uint32_t)sizeof(GenView) : 0u));
+        if constexpr (MATRIX) dev::bulk_load(&gstage[s], P.gen + v, (uint32_t)sizeof(GenView), &full[s]);
         dev::tma_load_3d(smem_raw + (size_t)s * stage_bytes, &tmap, &full[s], w0, h0, P.view0 + v);
         issued++;
         if (++ps == P.stages) { ps = 0; pround ^= 1u; }
@@ -555,6 +608,41 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
     const int4 org = origin[s];
     const int v = PIW ? org.z : j;
     if (PIW && v < 0) break;
+    if constexpr (MATRIX) {
+      MatrixColumn c = matrix_column(gstage[s], x, y, zf, NZ, P.wexp, org, P.BW, P.BH);
+      if (!c.ok) {  // memory safety: every tap must stay inside the staged box
+        dev::record_status(P.status, DEV_RANGE);
+        c.iw = 0; c.mv = 0.0f; c.bv = __int_as_float(org.y); c.rs = 1.0f; c.wt = 0.0f;
+      }
+      const uint32_t base = smem_base + (uint32_t)s * (uint32_t)stage_bytes + (uint32_t)c.iw * ESC -
+                            (MAGIC_BITS + (uint32_t)(int)__int_as_float(org.y)) * rowb;
+      const u64 MAG2 = pk2(MAGIC, MAGIC), FW2 = pk2(c.fw, c.fw), WT2 = pk2(c.wt, c.wt);
+      const u64 MV2 = pk2(c.mv, c.mv), BV2 = pk2(c.bv, c.bv), RS2 = pk2(c.rs, c.rs), TWO2 = pk2(2.0f, 2.0f);
+      u64 Z = pk2(zf, zf + 1.0f);
+#pragma unroll
+      for (int k = 0; k < NACC; k++) {
+        const u64 H = mul2(fma2(MV2, Z, BV2), RS2);
+        const u64 T2 = add2_rm(H, MAG2);
+        const u64 FH = sub2(H, sub2(T2, MAG2));
+        float t0, t1;
+        up2(T2, t0, t1);
+        const uint32_t a0 = (uint32_t)__float_as_uint(t0) * rowb + base;
+        const uint32_t a1 = (uint32_t)__float_as_uint(t1) * rowb + base;
+        const uint32_t c0 = a0 + rowb, c1 = a1 + rowb;
+        const u64 A = lds_f32x2<0>(a0, a1);
+        const u64 B = lds_f32x2<4>(a0, a1);
+        const u64 C = lds_f32x2<0>(c0, c1);
+        const u64 Dd = lds_f32x2<4>(c0, c1);
+        const u64 R0 = fma2(FW2, sub2(B, A), A);
+        const u64 R1 = fma2(FW2, sub2(Dd, C), C);
+        acc2[k] = fma2(WT2, fma2(FH, sub2(R1, R0), R0), acc2[k]);
+        Z = add2(Z, TWO2);
+      }
+      __syncwarp();
+      if (lane == 0) dev::mbar_arrive(&empty[s]);
+      if (++s == P.stages) { s = 0; ph ^= 1u; }
+      continue;
+    }
     const FdkView V = vstage[s];
 
     const float den = fmaf(V.c0, x, fmaf(V.c1, y, 1.0f));
@@ -714,7 +802,7 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
 //   consumers  --empty2[p] (one arrive per consumer warp)-->  producer
 // The producer itself frees a TMA stage once it has rewritten it.  The views it selects
 // (all, or with the PI window those that reach the tile) end with a marker buffer (view -1).
-template <typename T, int NZ, bool PIW>
+template <typename T, int NZ, bool PIW, bool MATRIX = false>
 __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_constant__ CUtensorMap tmap,
                                                                   const __grid_constant__ FdkParams P)
 {
@@ -729,7 +817,9 @@ __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_c
   int4* origin2 = reinterpret_cast<int4*>(pairs + (size_t)NP * pbuf_bytes);
   int4* sorg = origin2 + NP;
   FdkView* vpair = reinterpret_cast<FdkView*>(sorg + S);  // per pair buffer: its view's parameters
-  uint64_t* full = reinterpret_cast<uint64_t*>(vpair + NP);
+  static_assert(!MATRIX || !PIW, "matrix positions");
+  GenView* gpair = reinterpret_cast<GenView*>(vpair);     // MATRIX: the same
+  uint64_t* full = MATRIX ? reinterpret_cast<uint64_t*>(gpair + NP) : reinterpret_cast<uint64_t*>(vpair + NP);
   uint64_t* full2 = full + S;
   uint64_t* empty2 = full2 + NP;
 
@@ -824,8 +914,11 @@ __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_c
       }
       if (lane == 0) {
         origin2[p] = o;
-        vpair[p] = P.v[o.z];
+        if constexpr (!MATRIX) vpair[p] = P.v[o.z];
       }
+      if constexpr (MATRIX)
+        if (lane < (int)(sizeof(GenView) / sizeof(float4)))
+          reinterpret_cast<float4*>(gpair + p)[lane] = __ldg(reinterpret_cast<const float4*>(P.gen + o.z) + lane);
       __syncwarp();
       dev::mbar_arrive(&full2[p]);  // all 32 lanes: their writes are released to the consumers
       conv++;
@@ -881,6 +974,39 @@ __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_c
     const int4 org = origin2[p];
     const int v = org.z;
     if (v < 0) break;
+    if constexpr (MATRIX) {  // as in fdk_tma_kernel, from the tap-pair words
+      MatrixColumn c = matrix_column(gpair[p], x, y, zf, NZ, P.wexp, org, P.BW, P.BH);
+      if (!c.ok) {
+        dev::record_status(P.status, DEV_RANGE);
+        c.iw = 0; c.mv = 0.0f; c.bv = __int_as_float(org.y); c.rs = 1.0f; c.wt = 0.0f;
+      }
+      const uint32_t base = pair0 + (uint32_t)p * (uint32_t)pbuf_bytes + (uint32_t)c.iw * 4u -
+                            (MAGIC_BITS + (uint32_t)(int)__int_as_float(org.y)) * rowb;
+      const u64 MAG2 = pk2(MAGIC, MAGIC), FW2 = pk2(c.fw, c.fw), WT2 = pk2(c.wt, c.wt);
+      const u64 MV2 = pk2(c.mv, c.mv), BV2 = pk2(c.bv, c.bv), RS2 = pk2(c.rs, c.rs), TWO2 = pk2(2.0f, 2.0f);
+      u64 Z = pk2(zf, zf + 1.0f);
+#pragma unroll
+      for (int k = 0; k < NACC; k++) {
+        const u64 H = mul2(fma2(MV2, Z, BV2), RS2);
+        const u64 T2 = add2_rm(H, MAG2);
+        const u64 FH = sub2(H, sub2(T2, MAG2));
+        float t0, t1;
+        up2(T2, t0, t1);
+        const uint32_t a0 = (uint32_t)__float_as_uint(t0) * rowb + base;
+        const uint32_t a1 = (uint32_t)__float_as_uint(t1) * rowb + base;
+        u64 A, B, C, Dd;
+        lds_pair_taps<T>(a0, a1, A, B);
+        lds_pair_taps<T>(a0 + rowb, a1 + rowb, C, Dd);
+        const u64 R0 = fma2(FW2, sub2(B, A), A);
+        const u64 R1 = fma2(FW2, sub2(Dd, C), C);
+        acc2[k] = fma2(WT2, fma2(FH, sub2(R1, R0), R0), acc2[k]);
+        Z = add2(Z, TWO2);
+      }
+      __syncwarp();
+      if (lane == 0) dev::mbar_arrive(&empty2[p]);
+      if (++p == NP) { p = 0; ph ^= 1u; }
+      continue;
+    }
     const FdkView V = vpair[p];
     const float den = fmaf(V.c0, x, fmaf(V.c1, y, 1.0f));
     // the approximate reciprocal (within 2 ulp): the staging box keeps a pixel of margin
@@ -990,12 +1116,6 @@ namespace fcb {
 // Generic projective-matrix kernel
 // =====================================================================================
 constexpr int GEN_MAXV = 480;
-struct GenView {
-  float m[12];
-  float kappa;
-  float wt;
-  float wc, hc;  // local window column of the detector centre, row of the source (PI window)
-};
 struct GenParams {
   float* vol;
   const void* proj;
@@ -1164,6 +1284,24 @@ __global__ void pi_pairs_kernel(const PiView* __restrict__ views, int nviews, in
 }  // namespace fcb
 
 // =====================================================================================
+// Rows that TMA cannot describe
+// =====================================================================================
+// A tensor map wants a 16-byte aligned base and row strides of whole 16 bytes.  Projections of
+// other widths are copied, a launch's views at a time, to rows at a pitch that has them (the map
+// keeps the true width, so the padding is never read).  251 x 237 x 203 voxels, 200 views of
+// 379 x 231, on one B200: 2.02 ms with the copies and the matrix positions, 11.5 ms by the generic
+// kernel's global gathers (the same bits), 1.77 ms for rows of 380.
+namespace fcb {
+template <typename T>
+__global__ void repack_rows_kernel(const T* __restrict__ in, T* __restrict__ out, int W, int pitch, long long rows)
+{
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= W) return;
+  for (long long r = blockIdx.y; r < rows; r += gridDim.y) out[r * pitch + c] = in[r * W + c];
+}
+}  // namespace fcb
+
+// =====================================================================================
 // Plans
 // =====================================================================================
 using namespace fcb;
@@ -1182,9 +1320,11 @@ struct fcb_bp_plan {
   std::vector<GenParams> gen;
   std::vector<int> gen_parent;  // the view chunk (launch of `fdk`, or itself) each `gen` entry belongs to
   int4* d_win = nullptr;  // reference-compatible window table (device), when in use
+  GenView* d_gen = nullptr;  // rows that TMA cannot describe: the views' matrices (device)
   ~fcb_bp_plan()
   {
     if (d_win) cudaFree(d_win);
+    if (d_gen) cudaFree(d_gen);
   }
 };
 
@@ -1192,20 +1332,20 @@ namespace {
 
 // Dynamic shared memory of one fdk_tma_kernel CTA: `stages` boxes of BW x BH elements of
 // `es` bytes, a full and an empty barrier and a footprint record per stage.
-size_t fdk_smem_bytes(int BW, int BH, int stages, size_t es)
+size_t fdk_smem_bytes(int BW, int BH, int stages, size_t es, size_t record = sizeof(FdkView))
 {
   const size_t stage_bytes = ((size_t)BW * BH * es + 127) & ~(size_t)127;
-  return stages * stage_bytes + stages * (2 * sizeof(uint64_t) + sizeof(int4) + sizeof(FdkView));
+  return stages * stage_bytes + stages * (2 * sizeof(uint64_t) + sizeof(int4) + record);
 }
 
 // Dynamic shared memory of one fdk_pair_kernel CTA: `stages` boxes of 16-bit taps, `pbufs`
 // tap-pair buffers of BW x BH words, their footprint records and barriers.
-size_t fdk_pair_smem_bytes(int BW, int BH, int stages, int pbufs)
+size_t fdk_pair_smem_bytes(int BW, int BH, int stages, int pbufs, size_t record = sizeof(FdkView))
 {
   const size_t stage_bytes = ((size_t)BW * BH * 2 + 127) & ~(size_t)127;
   const size_t pbuf_bytes = ((size_t)BW * BH * 4 + 127) & ~(size_t)127;
   return stages * stage_bytes + pbufs * pbuf_bytes + (size_t)(stages + pbufs) * sizeof(int4) +
-         (size_t)pbufs * sizeof(FdkView) + (size_t)(stages + 2 * pbufs) * sizeof(uint64_t);
+         (size_t)pbufs * record + (size_t)(stages + 2 * pbufs) * sizeof(uint64_t);
 }
 
 // Launches chunk `chunk` (-1: all) over the z-tile layers [tz0, tz1) of the plan.
@@ -1248,6 +1388,69 @@ int launch_fdk_pair(fcb_bp_plan* pl, const CUtensorMap& map, int chunk, int tz0,
   return FCB_OK;
 }
 
+// Launches one chunk (P: its parameters, views at 0 .. nviews of the map) with matrix positions.
+template <typename T>
+int launch_matrix(const fcb_bp_plan* pl, const CUtensorMap& map, const FdkParams& P, int ntiles, cudaStream_t st)
+{
+  if constexpr (sizeof(T) == 4) {
+    const size_t smem = fdk_smem_bytes(pl->BW, pl->BH, pl->stages, sizeof(T), sizeof(GenView));
+    auto kern = fdk_tma_kernel<float, 32, false, true, 3, true>;
+    FCB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<ntiles, FDK_THREADS, smem, st>>>(map, P);
+  } else {
+    const size_t smem = fdk_pair_smem_bytes(pl->BW, pl->BH, pl->stages, pl->pbufs, sizeof(GenView));
+    auto kern = fdk_pair_kernel<T, 32, false, true>;
+    FCB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<ntiles, FDK_THREADS, smem, st>>>(map, P);
+  }
+  FCB_CUDA_TRY(cudaGetLastError());
+  return FCB_OK;
+}
+
+CUtensorMapDataType tmap_type(int ptype)
+{
+  return ptype == FCB_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+         : ptype == FCB_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                            : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+}
+
+// The staged kernels on projections whose rows TMA cannot describe: each launch's views copied to
+// rows of whole 16 bytes in stream-ordered scratch.  *done == false: no scratch to be had.
+template <typename T>
+int execute_repacked(fcb_bp_plan* pl, int chunk, int tz0, int tz1, const void* proj, float* volume, cudaStream_t st,
+                     bool* done)
+{
+  *done = false;
+  const int W = pl->pb.projWHSize[0], H = pl->pb.projWHSize[1], es = (int)sizeof(T);
+  const int pitch = (W * es + 15) / 16 * 16 / es;
+  int maxv = 0;
+  for (const FdkParams& F : pl->fdk) maxv = std::max(maxv, F.nviews);
+  void* buf = nullptr;
+  if (scratch_alloc(&buf, (size_t)maxv * H * pitch * es, st) != FCB_OK) return ok();
+  int rc = FCB_OK;
+  for (int c = 0; c < (int)pl->fdk.size() && rc == FCB_OK; c++) {
+    const FdkParams& F = pl->fdk[c];
+    const int layer = F.tiles_x * F.tiles_y, ntiles = (tz1 - tz0) * layer;
+    if ((chunk >= 0 && c != chunk) || ntiles <= 0) continue;
+    const long long rows = (long long)F.nviews * H;
+    repack_rows_kernel<T><<<dim3((unsigned)((W + 127) / 128), (unsigned)std::min<long long>(rows, 16384)), 128, 0, st>>>(
+        reinterpret_cast<const T*>(proj) + (size_t)F.view0 * H * W, reinterpret_cast<T*>(buf), W, pitch, rows);
+    CUtensorMap map;
+    rc = encode_tmap_3d(&map, tmap_type(pl->ptype), buf, W, H, F.nviews, (uint64_t)pitch * es,
+                        (uint64_t)pitch * H * es, pl->BW, pl->BH, 1);
+    if (rc) break;
+    FdkParams P = F;
+    P.vol = volume;
+    P.tile0 = tz0 * layer;
+    P.gen = pl->d_gen + F.view0;
+    P.view0 = 0;
+    rc = launch_matrix<T>(pl, map, P, ntiles, st);
+  }
+  scratch_free(buf, st);
+  *done = true;
+  return rc;
+}
+
 bool aligned_geometry(const Problem& pb) { return !pb.misaligned; }
 
 // Fill FdkParams for views [v0, v0+n) (sizes/box filled by the caller).
@@ -1272,17 +1475,17 @@ void fill_fdk_views(const Problem& pb, int mode, int v0, int n, FdkParams* P)
 }
 
 // Fill GenParams views [v0, v0+n): projective matrices, weights, window centre and source row.
-void fill_gen_views(const Problem& pb, int v0, int n, GenParams* P)
+void fill_gen_views(const Problem& pb, int v0, int n, GenView* out)
 {
   for (int k = 0; k < n; k++) {
     const int t = v0 + k;
     double M[12], kappa;
     view_matrix(pb, t, M, &kappa);
-    for (int j = 0; j < 12; j++) P->v[k].m[j] = (float)M[j];
-    P->v[k].kappa = (float)kappa;
-    P->v[k].wt = (float)pb.norm[t];
-    P->v[k].wc = (float)(pb.projDim[0] / 2 - pb.woff[t]);
-    P->v[k].hc = (float)(pb.projDim[1] / 2 - pb.hoff[t]);
+    for (int j = 0; j < 12; j++) out[k].m[j] = (float)M[j];
+    out[k].kappa = (float)kappa;
+    out[k].wt = (float)pb.norm[t];
+    out[k].wc = (float)(pb.projDim[0] / 2 - pb.woff[t]);
+    out[k].hc = (float)(pb.projDim[1] / 2 - pb.hoff[t]);
   }
 }
 
@@ -1486,6 +1689,19 @@ static int bp_plan_build(const fcb_geometry* g, int kernelMode, int projType, in
         P.status = scratch;
       }
   }
+  if (pl->path == 1 && may_alloc && !piwin && pl->nz_tile == 32 &&
+      ((size_t)pb.projWHSize[0] * dtype_size(projType)) % 16 != 0) {
+    // rows that TMA cannot describe: the matrices that the staged kernels then take positions from
+    std::vector<GenView> gv((size_t)pb.nviews);
+    fill_gen_views(pb, 0, pb.nviews, gv.data());
+    if (cudaMalloc(&pl->d_gen, gv.size() * sizeof(GenView)) != cudaSuccess) {
+      cudaGetLastError();
+      pl->d_gen = nullptr;  // the generic kernel needs none
+    } else if (cudaMemcpy(pl->d_gen, gv.data(), gv.size() * sizeof(GenView), cudaMemcpyHostToDevice) != cudaSuccess) {
+      delete pl;
+      return set_error(FCB_ERR_CUDA, "copy of the view matrices failed");
+    }
+  }
   if (pl->path == 0) {
     const int gmax = std::min(GEN_MAXV, pl->maxv);
     for (int v0 = 0; v0 < pb.nviews; v0 += gmax) {
@@ -1500,7 +1716,7 @@ static int bp_plan_build(const fcb_geometry* g, int kernelMode, int projType, in
       P.view0 = v0;
       P.piwin = piwin ? 1 : 0;
       P.td_a = td_a; P.td_r = td_r; P.td_sign = td_sign;
-      fill_gen_views(pb, v0, P.nviews, &P);
+      fill_gen_views(pb, v0, P.nviews, P.v);
       if (compat) {
         P.win = pl->d_win;
         P.sv0 = rw.subVolDim[0]; P.sv1 = rw.subVolDim[1]; P.sv2 = rw.subVolDim[2];
@@ -1549,10 +1765,7 @@ int bp_plan_execute_range(fcb_bp_plan* pl, int chunk, int z0, int z1, const void
                 ((size_t)pb.projWHSize[0] * es) % 16 == 0;
   if (pl->path == 1 && tma_ok) {
     CUtensorMap map;
-    const CUtensorMapDataType dt = pl->ptype == FCB_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
-                                   : pl->ptype == FCB_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
-                                                          : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    FCB_TRY(encode_tmap_3d(&map, dt, const_cast<void*>(proj), pb.projWHSize[0], pb.projWHSize[1],
+    FCB_TRY(encode_tmap_3d(&map, tmap_type(pl->ptype), const_cast<void*>(proj), pb.projWHSize[0], pb.projWHSize[1],
                            pb.nviews, (uint64_t)pb.projWHSize[0] * es,
                            (uint64_t)pb.projWHSize[0] * pb.projWHSize[1] * es, pl->BW, pl->BH, 1));
     for (FdkParams& P : pl->fdk) P.vol = volume;
@@ -1603,6 +1816,18 @@ int bp_plan_execute_range(fcb_bp_plan* pl, int chunk, int z0, int z1, const void
     }
     return ok();
   }
+  if (pl->path == 1 && pl->d_gen && (uintptr_t)proj % es == 0) {
+    // (not under capture: the scratch would become part of the graph)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    FCB_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+    bool done = false;
+    if (cap == cudaStreamCaptureStatusNone) {
+      if (pl->ptype == FCB_F32) FCB_TRY(execute_repacked<float>(pl, chunk, tz0, tz1, proj, volume, st, &done));
+      else if (pl->ptype == FCB_F16) FCB_TRY(execute_repacked<__half>(pl, chunk, tz0, tz1, proj, volume, st, &done));
+      else FCB_TRY(execute_repacked<__nv_bfloat16>(pl, chunk, tz0, tz1, proj, volume, st, &done));
+    }
+    if (done) return ok();
+  }
   if (pl->gen.empty()) {
     // TMA path planned but this buffer cannot be described by a descriptor: build the
     // generic parameters on the fly, each staged launch's views in pieces of at most
@@ -1623,7 +1848,7 @@ int bp_plan_execute_range(fcb_bp_plan* pl, int chunk, int z0, int z1, const void
         P.td_a = F.td_a;
         P.td_r = F.td_r;
         P.td_sign = F.td_sign;
-        fill_gen_views(pb, v0, P.nviews, &P);
+        fill_gen_views(pb, v0, P.nviews, P.v);
         pl->gen_parent.push_back(fc);
         pl->gen.push_back(P);
       }
