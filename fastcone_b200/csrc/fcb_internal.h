@@ -118,6 +118,16 @@ int encode_tmap_3d(CUtensorMap* map, CUtensorMapDataType dtype, void* base, uint
 int encode_tmap(CUtensorMap* map, CUtensorMapDataType dtype, int rank, void* base,
                 const uint64_t* dims, const uint64_t* strides_bytes, const uint32_t* box);
 
+// Lets a kernel without static shared memory use all that a CTA can have.  The limit is the
+// kernel's, not the launch's: set to each launch's own size, a launch of another thread that needs
+// more could find it lowered between its own setting and its launch.
+template <typename Kern>
+int allow_dynamic_smem(Kern kern)
+{
+  FCB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+  return FCB_OK;
+}
+
 inline int dtype_size(int t) { return t == FCB_F32 ? 4 : 2; }
 
 }  // namespace fcb

@@ -909,8 +909,7 @@ int brick_launch(std::vector<PjParams>& chunks, const BrickSetup& bs, const floa
   auto pkern = bs.T == 12  ? (bs.minb == 3 ? project_brick_kernel<3, 12> : project_brick_kernel<1, 12>)
                : bs.T == 8 ? (bs.minb == 3 ? project_brick_kernel<3, 8> : project_brick_kernel<1, 8>)
                            : (bs.minb == 3 ? project_brick_kernel<3, 6> : project_brick_kernel<1, 6>);
-  FCB_CUDA_TRY(cudaFuncSetAttribute(pkern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)bs.smem));
+  FCB_TRY(allow_dynamic_smem(pkern));
   for (PjParams& P : chunks) {
     P.BC = bs.BC;
     P.BZ = bs.BZ;
@@ -943,7 +942,7 @@ int brick_adjoint_launch(std::vector<PjParams>& chunks, const BrickSetup& bs, fl
   auto kern = bs.T == 12  ? (m4 ? project_adjoint_brick_kernel<4, 12> : project_adjoint_brick_kernel<5, 12>)
               : bs.T == 8 ? (m4 ? project_adjoint_brick_kernel<4, 8> : project_adjoint_brick_kernel<5, 8>)
                           : (m4 ? project_adjoint_brick_kernel<4, 6> : project_adjoint_brick_kernel<5, 6>);
-  FCB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  FCB_TRY(allow_dynamic_smem(kern));
   for (PjParams& P : chunks) {
     P.BC = bs.BC;
     P.BZ = bs.BZ;
