@@ -434,12 +434,89 @@ __device__ __forceinline__ MatrixColumn matrix_column(const GenView& V, float x,
   return c;
 }
 
+// SPLIT: the views of a tile shared by the CTAs of a cluster (rank r takes the r-th part of them),
+// for volumes whose tiles alone leave the chip idle.  Each CTA leaves its sums in its own shared
+// memory, rank r adds the r-th part of the tile's planes over the ranks, in rank order (the result
+// does not depend on timing), and adds them to the volume.  Every thread of the cluster meets both
+// cluster barriers, a CTA whose bounded waits ran out included, so they complete and nobody reads
+// the memory of a CTA that is gone.
+__device__ __forceinline__ uint32_t cluster_rank()
+{
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_size()
+{
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync()
+{
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+// views [*v0, *v1) of rank r among s
+__device__ __forceinline__ void split_views(int nviews, uint32_t r, uint32_t s, int* v0, int* v1)
+{
+  *v0 = (int)((long long)nviews * r / s);
+  *v1 = (int)((long long)nviews * (r + 1) / s);
+}
+// acc: the thread's NACC plane pairs.  Called by the consumer warps (256 threads); the producer warp
+// meets the two cluster barriers on its own.
+constexpr int SPLIT_SUMS = 32 * FDK_CWARPS * 32 * (int)sizeof(float);  // a tile's sums, over the staged boxes
+template <int NACC>
+__device__ __forceinline__ void split_store(unsigned char* smem_raw, const u64 (&acc)[NACC], const FdkParams& P, int xl,
+                                            int yl, int zl)
+{
+  static_assert(2 * NACC * FDK_CWARPS * 32 * (int)sizeof(float) <= SPLIT_SUMS, "sums of a tile");
+  const int tid = threadIdx.x;
+  float* sums = reinterpret_cast<float*>(smem_raw);  // [2 NACC][256]
+  __syncwarp();
+  asm volatile("bar.sync 1, %0;" ::"n"(FDK_CWARPS * 32) : "memory");  // every warp is done with them
+#pragma unroll
+  for (int k = 0; k < NACC; k++) {
+    float v0, v1;
+    up2(acc[k], v0, v1);
+    sums[(2 * k) * 256 + tid] = v0;
+    sums[(2 * k + 1) * 256 + tid] = v1;
+  }
+  cluster_sync();
+  const uint32_t rank = cluster_rank(), n = cluster_size();
+  const int z0 = 2 * NACC * (int)rank / (int)n, z1 = 2 * NACC * ((int)rank + 1) / (int)n;
+  const uint32_t mine = dev::smem_u32(sums) + (uint32_t)tid * 4u;
+  if (xl < P.nx && yl < P.ny) {
+    float* out = P.vol + (size_t)yl * P.nx + xl;
+    const size_t plane = (size_t)P.nx * P.ny;
+#pragma unroll 2
+    for (int z = z0; z < z1; z++) {
+      if (zl + z >= P.nz) break;
+      float w[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) {  // (remote loads of all ranks in flight)
+        if (q >= (int)n) break;
+        uint32_t a;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(mine + (uint32_t)z * 1024u), "r"(q));
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(w[q]) : "r"(a) : "memory");
+      }
+      float v = w[0];
+#pragma unroll
+      for (int q = 1; q < 8; q++)
+        if (q < (int)n) v += w[q];
+      out[(size_t)(zl + z) * plane] += v;
+    }
+  }
+  cluster_sync();  // the sums stay until every rank has read them
+}
+
 // Resident CTAs per SM the register allocation must allow: 3 (the default 64 KB staging
 // budget fits 3 CTAs) unless NZ = 64 needs the registers of 2.
 template <int NZ>
 constexpr int fdk_min_blocks() { return NZ >= 64 ? 2 : 3; }
 
-template <typename T, int NZ, bool PIW, bool X2, int MINB = fdk_min_blocks<NZ>(), bool MATRIX = false>
+template <typename T, int NZ, bool PIW, bool X2, int MINB = fdk_min_blocks<NZ>(), bool MATRIX = false,
+          bool SPLIT = false>
 __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid_constant__ CUtensorMap tmap,
                                                               const __grid_constant__ FdkParams P)
 {
@@ -451,7 +528,8 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
   constexpr int ESC = ES;  // bytes per position of the box the taps are read from
   const int stage_elems = P.BW * P.BH;
   const int stage_bytes = ((stage_elems * ES) + 127) & ~127;
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + (size_t)P.stages * stage_bytes);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + (SPLIT ? max(P.stages * stage_bytes, SPLIT_SUMS)
+                                                                 : P.stages * stage_bytes));
   uint64_t* empty = full + P.stages;
   // per stage: box origin w, h (as float bits: the consumers use them as floats); view (-1:
   // end of the list); rows the tile's footprint needs
@@ -466,7 +544,11 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int tx, ty, tz;
-  fdk_tile(P, P.tile0 + blockIdx.x, tx, ty, tz);
+  static_assert(!SPLIT || X2, "split views");
+  const uint32_t rank = SPLIT ? cluster_rank() : 0, nrank = SPLIT ? cluster_size() : 1;
+  fdk_tile(P, P.tile0 + (SPLIT ? blockIdx.x / nrank : blockIdx.x), tx, ty, tz);
+  int v0 = 0, v1 = P.nviews;  // this CTA's views (PI window: every nrank-th batch of 32)
+  if constexpr (SPLIT && !PIW) split_views(P.nviews, rank, nrank, &v0, &v1);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < P.stages; s++) {
@@ -477,8 +559,8 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
   }
   __syncthreads();
 
-  if (warp == FDK_CWARPS) {
-    // ------------------------------------------------------------- producer warp
+  // ------------------------------------------------------------- producer warp
+  auto produce = [&]() {
     const uint32_t bytes = (uint32_t)(stage_elems * ES);
     int issued = 0;  // staged views so far
     int ps = 0;      // its ring slot (issued mod stages), kept by increments: no division
@@ -488,7 +570,7 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
       // the whole warp tests 32 views at a time against the PI window (most views miss a
       // tile of a helical scan); lane 0 stages the ones that reach it, in view order
       if (lane == 0) dev::tma_prefetch(&tmap);
-      for (int vb = 0; vb < P.nviews && !failed && !stalled; vb += 32) {
+      for (int vb = 32 * (int)rank; vb < P.nviews && !failed && !stalled; vb += 32 * (int)nrank) {
         const int v = vb + lane;
         int w0 = 0, h0 = 0, nw = 0, nh = 0;
         bool need = false;
@@ -533,8 +615,8 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
     } else {
       if (lane != 0) return;
       dev::tma_prefetch(&tmap);
-      for (int v = 0; v < P.nviews; v++) {
-        if (v == P.stop_after) {  // test hook
+      for (int v = v0; v < v1; v++) {
+        if (issued == P.stop_after) {  // test hook
           stalled = true;
           break;
         }
@@ -573,6 +655,13 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
       for (int j = max(0, issued - P.stages); j < issued; j++)
         dev::mbar_wait(&full[j % P.stages], (j / P.stages) & 1, 100000000ull);
     }
+  };
+  if (warp == FDK_CWARPS) {
+    produce();
+    if constexpr (SPLIT) {
+      cluster_sync();
+      cluster_sync();
+    }
     return;
   }
 
@@ -600,9 +689,12 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
   // and the phase parity are kept by increments (no integer division per view)
   int s = 0;
   uint32_t ph = 0;
-  for (int j = 0; PIW || j < P.nviews; j++) {
-    if (!dev::mbar_wait(&full[s], ph, P.cwait_ns)) {
+  for (int j = v0; PIW || j < v1; j++) {
+    bool landed = dev::mbar_wait(&full[s], ph, P.cwait_ns);
+    if constexpr (SPLIT) landed = __all_sync(0xffffffffu, landed);  // the warp leaves the loop as one
+    if (!landed) {
       dev::record_status(P.status, DEV_TIMEOUT);
+      if constexpr (SPLIT) break;
       return;
     }
     const int4 org = origin[s];
@@ -766,6 +858,10 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
     if (++s == P.stages) { s = 0; ph ^= 1u; }
   }
 
+  if constexpr (SPLIT) {
+    split_store<NACC>(smem_raw, acc2, P, xl, yl, zl);
+    return;
+  }
   if (xl < P.nx && yl < P.ny) {
     float* out = P.vol + (size_t)yl * P.nx + xl;
     const size_t plane = (size_t)P.nx * P.ny;
@@ -802,7 +898,7 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
 //   consumers  --empty2[p] (one arrive per consumer warp)-->  producer
 // The producer itself frees a TMA stage once it has rewritten it.  The views it selects
 // (all, or with the PI window those that reach the tile) end with a marker buffer (view -1).
-template <typename T, int NZ, bool PIW, bool MATRIX = false>
+template <typename T, int NZ, bool PIW, bool MATRIX = false, bool SPLIT = false>
 __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_constant__ CUtensorMap tmap,
                                                                   const __grid_constant__ FdkParams P)
 {
@@ -814,7 +910,8 @@ __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_c
   const int pbuf_bytes = ((stage_elems * 4) + 127) & ~127;
   unsigned char* pairs = smem_raw + (size_t)S * stage_bytes;
   // box origins (w, h as float bits, view, rows needed): per pair buffer and per TMA stage
-  int4* origin2 = reinterpret_cast<int4*>(pairs + (size_t)NP * pbuf_bytes);
+  const int boxes = S * stage_bytes + NP * pbuf_bytes;
+  int4* origin2 = reinterpret_cast<int4*>(smem_raw + (SPLIT ? max(boxes, SPLIT_SUMS) : boxes));
   int4* sorg = origin2 + NP;
   FdkView* vpair = reinterpret_cast<FdkView*>(sorg + S);  // per pair buffer: its view's parameters
   static_assert(!MATRIX || !PIW, "matrix positions");
@@ -825,7 +922,16 @@ __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_c
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int tx, ty, tz;
-  fdk_tile(P, P.tile0 + blockIdx.x, tx, ty, tz);
+  const uint32_t rank = SPLIT ? cluster_rank() : 0, nrank = SPLIT ? cluster_size() : 1;
+  fdk_tile(P, P.tile0 + (SPLIT ? blockIdx.x / nrank : blockIdx.x), tx, ty, tz);
+  // this CTA's views, in batches of 32: a run of them, or (PI window, where few reach the tile)
+  // every nrank-th batch
+  int v0 = 0, v1 = P.nviews, vstep = 32;
+  if constexpr (SPLIT && !PIW) split_views(P.nviews, rank, nrank, &v0, &v1);
+  if constexpr (SPLIT && PIW) {
+    v0 = 32 * (int)rank;
+    vstep = 32 * (int)nrank;
+  }
 
   if (threadIdx.x == 0) {
     for (int k = 0; k < S; k++) dev::mbar_init(&full[k], 1);
@@ -837,12 +943,12 @@ __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_c
   }
   __syncthreads();
 
-  if (warp == FDK_CWARPS) {
-    // ------------------------------------------------------------- producer warp
+  // ------------------------------------------------------------- producer warp
+  auto produce = [&]() {
     if (lane == 0) dev::tma_prefetch(&tmap);
     const uint32_t bytes = (uint32_t)(stage_elems * 2);
     // views in order, 32 tested at a time (PI window: those that reach the tile)
-    int vb = -32;
+    int vb = v0 - vstep;
     unsigned msk = 0;
     int lw0 = 0, lh0 = 0, lnw = 0, lnh = 0;
     bool exhausted = false, stalled = false, failed = false;
@@ -855,14 +961,14 @@ __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_c
         return;
       }
       while (msk == 0) {
-        vb += 32;
-        if (vb >= P.nviews) {
+        vb += vstep;
+        if (vb >= v1) {
           exhausted = true;
           return;
         }
         const int v = vb + lane;
         bool need = false;
-        if (v < P.nviews) {
+        if (v < v1) {
           float fp[4];
           fdk_box_origin(P, P.v[v], tx, ty, tz, NZ, lw0, lh0, lnw, lnh, fp);
           need = PIW ? !fdk_tile_outside_window(P, P.v[v], fp[0], fp[1], fp[2], fp[3]) : true;
@@ -945,6 +1051,13 @@ __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_c
     } else if (lane == 0) {
       dev::record_status(P.status, DEV_TIMEOUT);
     }
+  };
+  if (warp == FDK_CWARPS) {
+    produce();
+    if constexpr (SPLIT) {
+      cluster_sync();
+      cluster_sync();
+    }
     return;
   }
 
@@ -967,8 +1080,11 @@ __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_c
   int p = 0;
   uint32_t ph = 0;
   for (;;) {
-    if (!dev::mbar_wait(&full2[p], ph, P.cwait_ns)) {
+    bool landed = dev::mbar_wait(&full2[p], ph, P.cwait_ns);
+    if constexpr (SPLIT) landed = __all_sync(0xffffffffu, landed);  // the warp leaves the loop as one
+    if (!landed) {
       dev::record_status(P.status, DEV_TIMEOUT);
+      if constexpr (SPLIT) break;
       return;
     }
     const int4 org = origin2[p];
@@ -1096,6 +1212,10 @@ __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_c
     if (++p == NP) { p = 0; ph ^= 1u; }
   }
 
+  if constexpr (SPLIT) {
+    split_store<NACC>(smem_raw, acc2, P, xl, yl, zl);
+    return;
+  }
   if (xl < P.nx && yl < P.ny) {
     float* out = P.vol + (size_t)yl * P.nx + xl;
     const size_t plane = (size_t)P.nx * P.ny;
@@ -1332,29 +1452,63 @@ namespace {
 
 // Dynamic shared memory of one fdk_tma_kernel CTA: `stages` boxes of BW x BH elements of
 // `es` bytes, a full and an empty barrier and a footprint record per stage.
-size_t fdk_smem_bytes(int BW, int BH, int stages, size_t es, size_t record = sizeof(FdkView))
+size_t fdk_smem_bytes(int BW, int BH, int stages, size_t es, size_t record = sizeof(FdkView), bool split = false)
 {
   const size_t stage_bytes = ((size_t)BW * BH * es + 127) & ~(size_t)127;
-  return stages * stage_bytes + stages * (2 * sizeof(uint64_t) + sizeof(int4) + record);
+  return std::max(stages * stage_bytes, split ? (size_t)SPLIT_SUMS : 0) + stages * (2 * sizeof(uint64_t) + sizeof(int4) + record);
 }
 
 // Dynamic shared memory of one fdk_pair_kernel CTA: `stages` boxes of 16-bit taps, `pbufs`
 // tap-pair buffers of BW x BH words, their footprint records and barriers.
-size_t fdk_pair_smem_bytes(int BW, int BH, int stages, int pbufs, size_t record = sizeof(FdkView))
+size_t fdk_pair_smem_bytes(int BW, int BH, int stages, int pbufs, size_t record = sizeof(FdkView), bool split = false)
 {
   const size_t stage_bytes = ((size_t)BW * BH * 2 + 127) & ~(size_t)127;
   const size_t pbuf_bytes = ((size_t)BW * BH * 4 + 127) & ~(size_t)127;
-  return stages * stage_bytes + pbufs * pbuf_bytes + (size_t)(stages + pbufs) * sizeof(int4) +
+  return std::max(stages * stage_bytes + pbufs * pbuf_bytes, split ? (size_t)SPLIT_SUMS : 0) +
+         (size_t)(stages + pbufs) * sizeof(int4) +
          (size_t)pbufs * record + (size_t)(stages + 2 * pbufs) * sizeof(uint64_t);
+}
+
+// Ranks that share a tile's views (1: none) for `ntiles` tiles and `nviews` views.  The chip holds
+// 444 CTAs, three per SM.  Clusters of six fill the SMs of a GPC best; below 40 tiles eight ranks
+// reach more SMs, up to 800 tiles two shorten the second wave, beyond that a tile alone is faster.
+// One B200, 180 views, FP32, milliseconds with 1, 2, 4, 6 and 8 ranks: 32 tiles (64^3) 0.191, 0.107,
+// 0.058, 0.058, 0.046; 108 tiles (96^3) 0.194, 0.155, 0.147, 0.124, 0.132; 256 tiles (128^3) 0.283,
+// 0.281, 0.275, 0.249, 0.283 (BF16 0.326, 0.313, 0.302, 0.273, 0.308); 500 tiles (160^3) 0.524,
+// 0.465, 0.492, 0.481, 0.530; 864 tiles (192^3) 0.766, 0.775, 0.807, 0.799, 0.898.
+int split_ranks(int ntiles, int nviews)
+{
+  if (const char* e = getenv("FCB_FDK_SPLIT")) return std::max(1, std::min(8, atoi(e)));  // tuning knob
+  const int s = ntiles >= 800 ? 1 : ntiles > 444 ? 2 : ntiles >= 40 ? 6 : 8;
+  return std::max(1, std::min(s, nviews / 8));
+}
+
+// One launch of a staged kernel: `split` ranks per tile in clusters of that many CTAs.
+template <typename Kern>
+int launch_staged(Kern kern, size_t smem, int ntiles, int split, const CUtensorMap& map, const FdkParams& P,
+                  cudaStream_t st)
+{
+  FCB_TRY(allow_dynamic_smem(kern));
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof cfg);
+  cfg.gridDim = dim3((unsigned)(ntiles * split));
+  cfg.blockDim = dim3(FDK_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)split;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = split > 1 ? 1 : 0;
+  FCB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, map, P));
+  return FCB_OK;
 }
 
 // Launches chunk `chunk` (-1: all) over the z-tile layers [tz0, tz1) of the plan.
 template <typename T, int NZ, bool PIW, bool X2, int MINB = fdk_min_blocks<NZ>()>
 int launch_fdk(fcb_bp_plan* pl, const CUtensorMap& map, int chunk, int tz0, int tz1, cudaStream_t st)
 {
-  const size_t smem = fdk_smem_bytes(pl->BW, pl->BH, pl->stages, sizeof(T));
-  auto kern = fdk_tma_kernel<T, NZ, PIW, X2, MINB>;
-  FCB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   for (int c = 0; c < (int)pl->fdk.size(); c++) {
     if (chunk >= 0 && c != chunk) continue;
     FdkParams& P = pl->fdk[c];
@@ -1362,8 +1516,17 @@ int launch_fdk(fcb_bp_plan* pl, const CUtensorMap& map, int chunk, int tz0, int 
     P.tile0 = tz0 * layer;
     const int ntiles = (tz1 - tz0) * layer;
     if (ntiles <= 0) continue;
-    kern<<<ntiles, FDK_THREADS, smem, st>>>(map, P);
-    FCB_CUDA_TRY(cudaGetLastError());
+    if constexpr (X2 && NZ == 32 && MINB == fdk_min_blocks<NZ>()) {
+      const int split = split_ranks(ntiles, P.nviews);
+      if (split > 1) {
+        FCB_TRY(launch_staged(fdk_tma_kernel<T, NZ, PIW, X2, MINB, false, true>,
+                              fdk_smem_bytes(pl->BW, pl->BH, pl->stages, sizeof(T), sizeof(FdkView), true), ntiles,
+                              split, map, P, st));
+        continue;
+      }
+    }
+    FCB_TRY(launch_staged(fdk_tma_kernel<T, NZ, PIW, X2, MINB>,
+                          fdk_smem_bytes(pl->BW, pl->BH, pl->stages, sizeof(T)), ntiles, 1, map, P, st));
   }
   return FCB_OK;
 }
@@ -1372,9 +1535,6 @@ int launch_fdk(fcb_bp_plan* pl, const CUtensorMap& map, int chunk, int tz0, int 
 template <typename T, bool PIW>
 int launch_fdk_pair(fcb_bp_plan* pl, const CUtensorMap& map, int chunk, int tz0, int tz1, cudaStream_t st)
 {
-  const size_t smem = fdk_pair_smem_bytes(pl->BW, pl->BH, pl->stages, pl->pbufs);
-  auto kern = fdk_pair_kernel<T, 32, PIW>;
-  FCB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   for (int c = 0; c < (int)pl->fdk.size(); c++) {
     if (chunk >= 0 && c != chunk) continue;
     FdkParams& P = pl->fdk[c];
@@ -1382,8 +1542,13 @@ int launch_fdk_pair(fcb_bp_plan* pl, const CUtensorMap& map, int chunk, int tz0,
     P.tile0 = tz0 * layer;
     const int ntiles = (tz1 - tz0) * layer;
     if (ntiles <= 0) continue;
-    kern<<<ntiles, FDK_THREADS, smem, st>>>(map, P);
-    FCB_CUDA_TRY(cudaGetLastError());
+    const int split = split_ranks(ntiles, P.nviews);
+    const size_t smem = fdk_pair_smem_bytes(pl->BW, pl->BH, pl->stages, pl->pbufs, sizeof(FdkView), split > 1);
+    if (split > 1)
+      FCB_TRY(launch_staged(fdk_pair_kernel<T, 32, PIW, false, true>, smem, ntiles, split, map, P,
+                            st));
+    else
+      FCB_TRY(launch_staged(fdk_pair_kernel<T, 32, PIW>, smem, ntiles, 1, map, P, st));
   }
   return FCB_OK;
 }
@@ -1392,19 +1557,20 @@ int launch_fdk_pair(fcb_bp_plan* pl, const CUtensorMap& map, int chunk, int tz0,
 template <typename T>
 int launch_matrix(const fcb_bp_plan* pl, const CUtensorMap& map, const FdkParams& P, int ntiles, cudaStream_t st)
 {
+  const int split = split_ranks(ntiles, P.nviews);
   if constexpr (sizeof(T) == 4) {
-    const size_t smem = fdk_smem_bytes(pl->BW, pl->BH, pl->stages, sizeof(T), sizeof(GenView));
-    auto kern = fdk_tma_kernel<float, 32, false, true, 3, true>;
-    FCB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<ntiles, FDK_THREADS, smem, st>>>(map, P);
+    const size_t smem = fdk_smem_bytes(pl->BW, pl->BH, pl->stages, sizeof(T), sizeof(GenView), split > 1);
+    if (split > 1)
+      return launch_staged(fdk_tma_kernel<float, 32, false, true, 3, true, true>, smem, ntiles,
+                           split, map, P, st);
+    return launch_staged(fdk_tma_kernel<float, 32, false, true, 3, true>, smem, ntiles, 1, map, P, st);
   } else {
-    const size_t smem = fdk_pair_smem_bytes(pl->BW, pl->BH, pl->stages, pl->pbufs, sizeof(GenView));
-    auto kern = fdk_pair_kernel<T, 32, false, true>;
-    FCB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<ntiles, FDK_THREADS, smem, st>>>(map, P);
+    const size_t smem = fdk_pair_smem_bytes(pl->BW, pl->BH, pl->stages, pl->pbufs, sizeof(GenView), split > 1);
+    if (split > 1)
+      return launch_staged(fdk_pair_kernel<T, 32, false, true, true>, smem, ntiles, split, map, P,
+                           st);
+    return launch_staged(fdk_pair_kernel<T, 32, false, true>, smem, ntiles, 1, map, P, st);
   }
-  FCB_CUDA_TRY(cudaGetLastError());
-  return FCB_OK;
 }
 
 CUtensorMapDataType tmap_type(int ptype)
@@ -1649,13 +1815,23 @@ static int bp_plan_build(const fcb_geometry* g, int kernelMode, int projType, in
     if (e != cudaSuccess) { delete pl; return set_error(FCB_ERR_CUDA, cudaGetErrorString(e)); }
     const int align = 1 << pl->wshift;
     pl->BW = ((h[0] + align - 1) / align) * align;
-    // FP32 boxes: a row pitch of 4 mod 8 words puts the same column of consecutive rows in
-    // different shared-memory banks (a multiple of 8 or 16 makes rows collide: at 48 the
-    // slab case ran 13 % slower than at 44)
-    if (projType == FCB_F32 && pl->BW % 8 == 0) pl->BW += 4;
     pl->BH = h[1] + 1;  // + 1: the inner z layers' corner floors (see fdk_footprint_kernel)
     if (pl->BW < align) pl->BW = align;
     if (pl->BH < 2) pl->BH = 2;
+    // FP32 boxes: the row pitch decides the bank conflicts, since the lanes of a warp (8 x 4
+    // columns) read a dozen columns of a few neighbouring rows.  At 12 to 20 mod 32 words those
+    // spread over the banks for every detector pitch from 0.5 to 1.6 voxels (1.0 to 1.25 wavefronts
+    // per load); next to a multiple of 32 they collide (1.2 to 2).  One B200, padded against the
+    // width as it comes: 256^3 / 90 views at pitch 1.0 (44 against 36 words) 0.876 ms against
+    // 0.953, at 0.6 (76 against 56) 0.993 against 1.34; 128^3 / 180 views at 0.5 (76 against 60)
+    // 0.314 ms against 0.404.  PI-window launches, bound by their window tests, keep the smaller
+    // box (helix: 56.2 ms at 36 words, 56.4 at 44), at 4 mod 8 words.
+    if (projType == FCB_F32 && piwin) {
+      if (pl->BW % 8 == 0) pl->BW += 4;
+    } else if (projType == FCB_F32) {
+      const int r = pl->BW % 32, pad = r < 12 ? 12 - r : r > 20 ? 44 - r : 0;
+      if (pl->BW + pad <= 256 && fdk_smem_bytes(pl->BW + pad, pl->BH, 2, 4) <= 100 * 1024) pl->BW += pad;
+    }
     // the largest dynamic shared memory a CTA of this device may opt into
     int smem_optin = 227 * 1024;  // sm_100
     if (cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, pl->device) !=

@@ -14,8 +14,11 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("mode", [0, 1, 2])
 @pytest.mark.parametrize("vol,det,views", [((33, 30, 27), (71, 48), 250), ((17, 40, 65), (53, 31), 21),
                                            ((64, 64, 32), (97, 50), 181), ((16, 16, 1), (33, 9), 1)])
-def test_repacked_rows_equal_generic(vol, det, views, mode, dtype):
+def test_repacked_rows_equal_generic(vol, det, views, mode, dtype, monkeypatch):
     import torch
+
+    # one CTA per tile: the generic kernel's order of additions over the views
+    monkeypatch.setenv("FCB_FDK_SPLIT", "1")
 
     from fastcone_b200 import ops
 
