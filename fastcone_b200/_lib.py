@@ -43,7 +43,7 @@ EXPORTED_SYMBOLS = [
     "fcb_bp_plan_create", "fcb_bp_plan_execute", "fcb_bp_plan_info", "fcb_bp_plan_destroy",
     "fcb_sync_status", "fcb_fdk_filter_device", "fcb_phantom_device",
     "fcb_backproject_device_noalloc", "fcb_katsevich_filter_device",
-    "fcb_conv3d16_device", "fcb_conv3d16_wgrad_device",
+    "fcb_conv3d16_device", "fcb_conv3d16_wgrad_device", "fcb_conv3d16_grad_prep_device",
     "fcb_proj_plan_create", "fcb_proj_plan_execute", "fcb_proj_plan_destroy",
     "fcb_reference_windows", "fcb_proj_plan_info",
     "fcb_filter_plan_create", "fcb_filter_plan_create_ex", "fcb_filter_plan_execute",
@@ -126,6 +126,8 @@ def lib():
                                               ctypes.c_int, ctypes.c_int, vp]
             L.fcb_conv3d16_wgrad_device.argtypes = [vp, vp, ctypes.c_int, vp, ctypes.c_int, ctypes.c_int,
                                                     ctypes.c_int, vp]
+            L.fcb_conv3d16_grad_prep_device.argtypes = [vp, ctypes.c_int, vp, vp, vp, vp, ctypes.c_int,
+                                                        ctypes.c_int, ctypes.c_int, vp]
             L.fcb_katsevich_filter_device.argtypes = [vp, vp, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                                       c_float_p, ctypes.c_float, ctypes.c_float,
                                                       ctypes.c_float, ctypes.c_int, vp]

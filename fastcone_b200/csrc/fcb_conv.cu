@@ -15,7 +15,7 @@
 // ReLU and store.
 //
 // The same kernels compute the input gradient (transposed, tap-flipped weights, prepared by
-// the caller); conv3d16r_kernel (row reuse) is the default form.  The weight gradient, a
+// the caller); conv3d16n_kernel is the default form.  The weight gradient, a
 // 6912-entry reduction over all voxels, runs on the tensor cores too
 // (conv3d16_wgrad_tc_kernel, BF16 dY) with a CUDA-core kernel for FP32 dY and comparison.
 #include <stdlib.h>
@@ -73,6 +73,16 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16])
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// zeros into 32 lanes x 16 consecutive 32-bit columns
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr)
+{
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(
+                   taddr),
+               "r"(0u)
+               : "memory");
+}
+
 // Shared-memory matrix descriptor, K-major, no swizzle ("interleaved" core matrices of 8
 // rows x 16 bytes): start address, leading byte offset (between the two 8-element K
 // halves), stride byte offset (between 8-row groups), descriptor version 1 (sm_100).
@@ -118,7 +128,7 @@ constexpr int CV_SMEM = CV_A_BYTES + CV_W_BYTES + 64 + 32 + 16;
 
 struct ConvParams {
   int pairs;               // 1: boxes of voxel pairs (32-byte rows, even nx), 0: single voxels
-  uint32_t box_bytes;      // bytes of one staged half-row box
+  uint32_t box_bytes;      // bytes of one TMA box
   const __nv_bfloat16* w;  // [27][16 out][16 in]
   const float* bias;       // [16] or null
   void* out;               // [z][y][x][16], bf16 or f32
@@ -423,56 +433,90 @@ __global__ void __launch_bounds__(CVP_THREADS, 1) conv3d16p_kernel(const __grid_
   }
 }
 
-// Row-reusing form (default): a CTA walks chunks of CVR_YCH consecutive y rows of one
-// (x tile, z) column.  Neighbouring tiles share two of their three dy rows, so the input rows
-// live in a ring of 4 slots per dz (slot dz * 4 + (row & 3)) and each tile loads only its 3
-// new rows (9 at the start of a chunk): a third of the row traffic of conv3d16p_kernel.
-//   warp 4 (one lane): TMA producer; before refilling the slots of row y+1 it waits for
-//                      the MMAs of tile y-2, the last reader of the row it replaces;
-//   warp 5 (one lane): MMA issuer (27 MMAs per tile, taps addressed through the ring),
-//                      commits to the tile's done barrier and to the accumulator barrier;
-//   warps 0-3:         epilogue, as in conv3d16p_kernel.
-constexpr int CVR_YCH = 32;                 // rows per chunk
-constexpr int CVR_SLOTS = 12;               // 3 dz x 4 ring positions
-constexpr int CVR_THREADS = 192;
-constexpr int CVR_SMEM = CVR_SLOTS * 2 * CV_RB + CV_W_BYTES + 64 + 8 * (4 + 4 + 2 + 2) + 16;
+// The default form.  An MMA of N = 16 reads its 4 KB of A from shared memory for 8 cycles' worth of
+// arithmetic, so the kernels above are bound by operand reads and a fixed cost per MMA (27 per tile
+// at about 53 cycles).  Here one MMA covers the three dy taps: an input row contributes to the
+// output rows above, at and below it, whose accumulators lie side by side in tensor memory, so one
+// A row (per dz and dx) times the three taps' weights (N = 48) updates all three.  Nine MMAs per
+// row instead of 27, and every staged row is used once.
+// A CTA walks chunks of up to CVN_Y output rows of one (x tile, z) column, dz by dz, so that every
+// output gathers its taps in the order dz, dy, dx of the kernels above: the same bits (and the same
+// signs around zero, which a ReLU's gradient passes on).  Output row p of a chunk owns TMEM columns
+// 16 p .. 16 p + 15.  Input row i (y0 - 1 + i) updates rows i - 2, i - 1, i of those the chunk has;
+// with dz = 2 it completes row i - 2.
+//   warp 4 (one lane): TMA producer, CVN_G consecutive input rows per stage, one box each (a wait
+//                      and a commit per row cost as much as the row's MMAs: 0.500 ms);
+//   warp 5 (one lane): MMA issuer; commits free the stage and hand finished rows over;
+//   warps 0-3:         epilogue: read their TMEM lane quadrant of a finished row, clear it for the
+//                      next chunk (accumulators start from zero: rows join at different MMAs),
+//                      release it, then bias / ReLU / store.
+// 256^3 on one B200: 0.442 ms per layer, 0.646 with N = 16 and row reuse (HBM floor 0.165).  The
+// operand reads of an MMA take 44 cycles of shared memory; here one takes 97, since three MMAs on
+// one accumulator are followed by three on one that overlaps it (with nine in a row, the taps in
+// another order, 0.318).  Twice as many epilogue warps changed nothing.
+constexpr int CVN_Y = 16;
+constexpr int CVN_G = 3;                   // input rows per stage
+constexpr int CVN_STAGES = 5;
+constexpr int CVN_THREADS = 192;
+constexpr int CVN_STAGE = CVN_G * 2 * (CV_ROW + 2) * 16;  // [row][channel half][voxel] x 16 B
+constexpr int CVN_WB = 48 * 32;            // weights of one (dz, dx): [K half][dy = 2, 1, 0][16 out] x 16 B
+constexpr int CVN_COLS = 16 * CVN_Y;       // TMEM columns: two CTAs per SM
+constexpr int CVN_SMEM = CVN_STAGES * CVN_STAGE + 9 * CVN_WB + 64 + 8 * (2 * CVN_STAGES + 2 * CVN_Y) + 16;
+static_assert(CVN_STAGE % 128 == 0 && 3 * CVN_SMEM > 227 * 1024 && 2 * CVN_SMEM < 225 * 1024 && 2 * CVN_COLS <= 512,
+              "two CTAs per SM");
 
-__global__ void __launch_bounds__(CVR_THREADS, 2) conv3d16r_kernel(const __grid_constant__ CUtensorMap xmap,
+// The chunks of a volume: c -> x tile, z, rows [y0, y1)
+struct ConvChunks {
+  int tiles_x, ny, ych;
+  __device__ __forceinline__ void at(int c, int& x0, int& z, int& y0, int& y1) const
+  {
+    const int yc = c % ych, col = c / ych;
+    x0 = (col % tiles_x) * CV_TILE;
+    z = col / tiles_x;
+    y0 = yc * CVN_Y;
+    y1 = min(ny, y0 + CVN_Y);
+  }
+};
+
+__global__ void __launch_bounds__(CVN_THREADS, 2) conv3d16n_kernel(const __grid_constant__ CUtensorMap xmap,
                                                                   const __grid_constant__ ConvParams P,
                                                                   int nchunks)
 {
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* A = smem;
-  unsigned char* Wsm = smem + CVR_SLOTS * 2 * CV_RB;
-  float* bias = reinterpret_cast<float*>(Wsm + CV_W_BYTES);
-  uint64_t* rows_full = reinterpret_cast<uint64_t*>(Wsm + CV_W_BYTES + 64);  // [4] per tile
-  uint64_t* tile_done = rows_full + 4;                                         // [4] per tile
-  uint64_t* accf = tile_done + 4;                                              // [2]
-  uint64_t* acce = accf + 2;                                                   // [2]
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(acce + 2);
+  unsigned char* Wsm = smem + CVN_STAGES * CVN_STAGE;
+  float* bias = reinterpret_cast<float*>(Wsm + 9 * CVN_WB);
+  uint64_t* full = reinterpret_cast<uint64_t*>(Wsm + 9 * CVN_WB + 64);
+  uint64_t* empty = full + CVN_STAGES;
+  uint64_t* accf = empty + CVN_STAGES;  // [CVN_Y] output row complete (MMA commit)
+  uint64_t* acce = accf + CVN_Y;        // [CVN_Y] output row read and cleared (4 epilogue warps)
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(acce + CVN_Y);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ych = (P.ny + CVR_YCH - 1) / CVR_YCH;
+  const ConvChunks CH{P.tiles_x, P.ny, (P.ny + CVN_Y - 1) / CVN_Y};
 
   if (threadIdx.x == 0) {
-    for (int q = 0; q < 4; q++) {
-      dev::mbar_init(&rows_full[q], 1);
-      dev::mbar_init(&tile_done[q], 1);
+    for (int q = 0; q < CVN_STAGES; q++) {
+      dev::mbar_init(&full[q], 1);
+      dev::mbar_init(&empty[q], 1);
     }
-    for (int b = 0; b < 2; b++) {
-      dev::mbar_init(&accf[b], 1);
-      dev::mbar_init(&acce[b], 4);
+    for (int p = 0; p < CVN_Y; p++) {
+      dev::mbar_init(&accf[p], 1);
+      dev::mbar_init(&acce[p], 4);
     }
     dev::fence_mbar_init();
   }
   if (warp == 5) {
-    tc::tmem_alloc(tslot, 32);
+    tc::tmem_alloc(tslot, CVN_COLS);
     tc::tmem_relinquish();
   }
+  // weights: (dz, dx), K half kh, dy block (2, 1, 0), out channel n: 16 bytes of 8 in-channels
   const uint4* wg = reinterpret_cast<const uint4*>(P.w);
   for (int i = threadIdx.x; i < 27 * 16 * 2; i += blockDim.x) {
     const int t = i / 32, n = (i / 2) % 16, kh = i % 2;
-    reinterpret_cast<uint4*>(Wsm + t * 512 + kh * 256 + n * 16)[0] = wg[(t * 16 + n) * 2 + kh];
+    const int dz = t / 9, dy = (t / 3) % 3, dx = t % 3;
+    reinterpret_cast<uint4*>(Wsm + (dz * 3 + dx) * CVN_WB + kh * (CVN_WB / 2) + ((2 - dy) * 16 + n) * 16)[0] =
+        wg[(t * 16 + n) * 2 + kh];
   }
   if (threadIdx.x < 16) bias[threadIdx.x] = P.bias ? P.bias[threadIdx.x] : 0.0f;
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -480,111 +524,117 @@ __global__ void __launch_bounds__(CVR_THREADS, 2) conv3d16r_kernel(const __grid_
   __syncthreads();
   tc::fence_after();
   const uint32_t taddr = *tslot;
-
-  // chunk c -> x tile, z, rows [y0, y1)
-  auto chunk_of = [&](int c, int& x0, int& z, int& y0, int& y1) {
-    const int yc = c % ych, col = c / ych;
-    x0 = (col % P.tiles_x) * CV_TILE;
-    z = col / P.tiles_x;
-    y0 = yc * CVR_YCH;
-    y1 = min(P.ny, y0 + CVR_YCH);
-  };
-  int last = -1;  // tiles this CTA handles, minus one (same count in every role)
-  for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
-    int x0, z, y0, y1;
-    chunk_of(c, x0, z, y0, y1);
-    last += y1 - y0;
+  const uint32_t lanes = (uint32_t)(warp * 32) << 16;
+  if (warp < 4) {
+    for (int p = 0; p < CVN_Y; p++) tc::tmem_zero16(taddr + lanes + (uint32_t)(16 * p));
+    tc::tmem_wait_st();
   }
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
 
   if (warp == 4) {
     // ---------------------------------------------------------------- TMA producer
     if (lane == 0) {
       dev::tma_prefetch(&xmap);
-      int i = 0, issued = 0;
+      int issued = 0, s = 0;
+      uint32_t ph = 0;
       bool failed = false;
       for (int c = blockIdx.x; c < nchunks && !failed; c += gridDim.x) {
         int x0, z, y0, y1;
-        chunk_of(c, x0, z, y0, y1);
-        for (int y = y0; y < y1; y++, i++) {
-          const bool start = y == y0;
-          // slots about to be refilled must be done with: tile i-2 (in a chunk) or every
-          // earlier tile (a new chunk replaces all rows)
-          const int wt = start ? i - 1 : i - 2;
-          if (wt >= 0 && !dev::mbar_wait(&tile_done[wt & 3], (wt >> 2) & 1)) {
+        CH.at(c, x0, z, y0, y1);
+        const int groups = (y1 - y0 + 2 + CVN_G - 1) / CVN_G;
+        for (int j = 0; j < 3 * groups; j++) {  // dz slowest; rows past the chunk's are read, not used
+          if (issued >= CVN_STAGES && !dev::mbar_wait(&empty[s], ph ^ 1u)) {
             dev::record_status(P.status, DEV_TIMEOUT);
             failed = true;
             break;
           }
-          const int r0 = start ? -1 : 1;  // new rows y + r0 .. y + 1
-          const int nrows = 3 * (2 - r0);
-          dev::mbar_arrive_expect_tx(&rows_full[i & 3], (uint32_t)nrows * 2u * P.box_bytes);
-          for (int dz = 0; dz < 3; dz++)
-            for (int dy = r0; dy <= 1; dy++) {
-              const int yy = y + dy;
-              unsigned char* slot = A + (dz * 4 + (yy & 3)) * 2 * CV_RB;
-              for (int kh = 0; kh < 2; kh++)
-                tc::tma_load_5d(slot + kh * CV_RB, &xmap, &rows_full[i & 3], 0,
-                                P.pairs ? (x0 >> 1) - 1 : x0 - 1, kh, yy, z + dz - 1);
-            }
-          issued = i + 1;
+          const int dz = j / groups, y = y0 - 1 + CVN_G * (j - dz * groups);
+          dev::mbar_arrive_expect_tx(&full[s], P.box_bytes);
+          tc::tma_load_5d(A + s * CVN_STAGE, &xmap, &full[s], 0, P.pairs ? (x0 >> 1) - 1 : x0 - 1, 0, y, z + dz - 1);
+          issued++;
+          if (++s == CVN_STAGES) { s = 0; ph ^= 1u; }
         }
       }
-      for (int j = max(0, issued - 4); j < issued; j++)
-        dev::mbar_wait(&rows_full[j & 3], (j >> 2) & 1, 100000000ull);
+      // no copy may still be landing in shared memory when the CTA leaves (bounded waits)
+      for (int j = max(0, issued - CVN_STAGES); j < issued; j++)
+        dev::mbar_wait(&full[j % CVN_STAGES], (j / CVN_STAGES) & 1, 100000000ull);
     }
   } else if (warp == 5) {
     // ---------------------------------------------------------------- MMA issuer
     if (lane == 0) {
       const uint32_t wbase = dev::smem_u32(Wsm), abase = dev::smem_u32(A);
-      constexpr uint32_t IDESC = tc::idesc_bf16(CV_TILE, 16);
-      int i = 0;
+      int s = 0;
+      uint32_t ph = 0;
+      uint32_t used = 0;  // bit p: parity of the uses of output row p so far
+      int stages = 0;     // stages issued
+      const uint32_t half = P.box_bytes / (2 * CVN_G);  // one channel half of one staged row
       bool failed = false;
       for (int c = blockIdx.x; c < nchunks && !failed; c += gridDim.x) {
         int x0, z, y0, y1;
-        chunk_of(c, x0, z, y0, y1);
-        for (int y = y0; y < y1; y++, i++) {
-          const int b = i & 1;
-          if (!dev::mbar_wait(&rows_full[i & 3], (i >> 2) & 1) ||
-              (i >= 2 && !dev::mbar_wait(&acce[b], ((i >> 1) - 1) & 1))) {
-            dev::record_status(P.status, DEV_TIMEOUT);
-            failed = true;
-            break;
+        CH.at(c, x0, z, y0, y1);
+        const int n = y1 - y0;
+        for (int dz = 0; dz < 3 && !failed; dz++)
+          for (int i0 = 0; i0 < n + 2; i0 += CVN_G) {
+            const int i1 = min(i0 + CVN_G, n + 2);
+            bool ok = dev::mbar_wait(&full[s], ph);
+            // with dz = 0 the chunk's rows join: their previous uses must have been read and cleared
+            if (dz == 0)
+              for (int i = i0; ok && i < min(i1, n); i++) ok = dev::mbar_wait(&acce[i], ((used >> i) & 1u) ^ 1u);
+            if (!ok) {
+              dev::record_status(P.status, DEV_TIMEOUT);
+              failed = true;
+              break;
+            }
+            tc::fence_after();
+            for (int i = i0; i < i1; i++) {
+              const int plo = max(i - 2, 0), phi = min(i, n - 1);
+              const uint32_t idesc = tc::idesc_bf16(CV_TILE, 16 * (phi - plo + 1));
+              const uint32_t d = taddr + (uint32_t)(16 * plo);
+              const uint32_t a0 = abase + s * CVN_STAGE + (i - i0) * 2 * half + P.pairs * 16;
+              const uint32_t b0 = wbase + dz * 3 * CVN_WB + (plo - (i - 2)) * 256;
+#pragma unroll
+              for (int dx = 0; dx < 3; dx++)
+                tc::mma_bf16(d, tc::smem_desc(a0 + dx * 16, half, 128),
+                             tc::smem_desc(b0 + dx * CVN_WB, CVN_WB / 2, 128), idesc, 1u);
+              if (dz == 2 && i >= 2) tc::mma_commit(&accf[i - 2]);
+            }
+            tc::mma_commit(&empty[s]);
+            stages++;
+            if (++s == CVN_STAGES) { s = 0; ph ^= 1u; }
           }
-          tc::fence_after();
-          for (int t = 0; t < 27; t++) {
-            const int dz = t / 9, dy = (t / 3) % 3, dx = t % 3;
-            const int slot = dz * 4 + ((y + dy - 1) & 3);
-            const uint64_t ad = tc::smem_desc(abase + slot * 2 * CV_RB + (dx + P.pairs) * 16, CV_RB, 128);
-            const uint64_t bd = tc::smem_desc(wbase + t * 512, 256, 128);
-            tc::mma_bf16(taddr + (uint32_t)(b * 16), ad, bd, IDESC, t > 0 ? 1u : 0u);
-          }
-          tc::mma_commit(&tile_done[i & 3]);
-          tc::mma_commit(&accf[b]);
-        }
+        if (!failed) used ^= (1u << n) - 1u;
       }
+      // every MMA issued must be complete before the columns are released: the last stage's commit
+      if (stages > 0) dev::mbar_wait(&empty[(stages - 1) % CVN_STAGES], ((stages - 1) / CVN_STAGES) & 1, 100000000ull);
     }
   } else {
     // ---------------------------------------------------------------- epilogue (warps 0-3)
-    int i = 0;
+    uint32_t used = 0;
     bool failed = false;
     for (int c = blockIdx.x; c < nchunks && !failed; c += gridDim.x) {
       int x0, z, y0, y1;
-      chunk_of(c, x0, z, y0, y1);
-      for (int y = y0; y < y1; y++, i++) {
-        const int b = i & 1;
-        if (!__all_sync(0xffffffffu, dev::mbar_wait(&accf[b], (i >> 1) & 1))) {
+      CH.at(c, x0, z, y0, y1);
+      const int n = y1 - y0;
+      const int xv = x0 + warp * 32 + lane;
+      for (int p = 0; p < n; p++) {
+        // warp-uniform: the tcgen05 instructions below are warp-collective
+        if (!__all_sync(0xffffffffu, dev::mbar_wait(&accf[p], (used >> p) & 1u))) {
           if (lane == 0) dev::record_status(P.status, DEV_TIMEOUT);
           failed = true;
           break;
         }
         tc::fence_after();
         uint32_t r[16];
-        tc::tmem_ld16(taddr + (uint32_t)(b * 16) + ((uint32_t)(warp * 32) << 16), r);
+        tc::tmem_ld16(taddr + lanes + (uint32_t)(16 * p), r);
+        tc::tmem_zero16(taddr + lanes + (uint32_t)(16 * p));
+        tc::tmem_wait_st();
         tc::fence_before();
         __syncwarp();
-        if (lane == 0) dev::mbar_arrive(&acce[b]);
-        const int xv = x0 + warp * 32 + lane;
+        if (lane == 0) dev::mbar_arrive(&acce[p]);
         if (xv < P.nx) {
+          const int y = y0 + p;
           float v[16];
 #pragma unroll
           for (int q = 0; q < 16; q++) {
@@ -612,15 +662,14 @@ __global__ void __launch_bounds__(CVR_THREADS, 2) conv3d16r_kernel(const __grid_
           }
         }
       }
+      used ^= (1u << n) - 1u;
     }
   }
-  // every MMA issued must be complete before the columns are released
-  if (warp == 5 && lane == 0 && last >= 0) dev::mbar_wait(&accf[last & 1], (last >> 1) & 1, 100000000ull);
   tc::fence_before();
   __syncthreads();
   if (warp == 5) {
     tc::fence_after();
-    tc::tmem_dealloc(taddr, 32);
+    tc::tmem_dealloc(taddr, CVN_COLS);
   }
 }
 
@@ -701,7 +750,7 @@ __global__ void __launch_bounds__(256) conv3d16_wgrad_kernel(const WgradParams P
 // pairs packed per 32-bit column) with tcgen05.st from the staged dY row; B is the staged X
 // rows, MN-major straight from the activation layout (8 channels of one voxel = one 16-byte
 // core-matrix row).  TMEM: 3 accumulators of 48 columns (144) + WGT_ABUF A buffers of 72.
-// A CTA walks chunks of CVR_YCH consecutive y rows of one (x tile, z) column; each tile loads
+// A CTA walks chunks of WGT_YCH consecutive y rows of one (x tile, z) column; each tile loads
 // its 3 new X rows into a ring of WGT_RING positions per dz, rows at positions 0 and 1 also
 // into positions WGT_RING and WGT_RING + 1, so that rows y-1, y, y+1 always occupy three
 // consecutive slots (a uniform N stride for B); dY rows are staged WGT_LEAD deep;
@@ -711,6 +760,7 @@ __global__ void __launch_bounds__(256) conv3d16_wgrad_kernel(const WgradParams P
 //   warp 3 (one lane): MMA issuer, commits to the tile's done barrier.
 // Dynamic shared memory above half an SM's keeps one CTA per SM (512-column allocation).
 constexpr int WGT_THREADS = 128;
+constexpr int WGT_YCH = 32;                          // rows per chunk
 constexpr int WGT_KSTEPS = 9;                        // 144 voxels u per tile
 constexpr int WGT_XROW = 148;                        // staged X voxels per row (from x0 - 2)
 constexpr int WGT_RB = 2432;                         // one channel half of a staged X row, 128-B multiple
@@ -761,7 +811,6 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
                "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                : "memory");
 }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 }  // namespace tc
 
 __global__ void __launch_bounds__(WGT_THREADS, 1) conv3d16_wgrad_tc_kernel(const __grid_constant__ CUtensorMap xmap,
@@ -780,7 +829,7 @@ __global__ void __launch_bounds__(WGT_THREADS, 1) conv3d16_wgrad_tc_kernel(const
   volatile int* failed_flag = reinterpret_cast<volatile int*>(tslot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ych = (P.ny + CVR_YCH - 1) / CVR_YCH;
+  const int ych = (P.ny + WGT_YCH - 1) / WGT_YCH;
 
   if (threadIdx.x == 0) {
     for (int q = 0; q < WGT_RING; q++) {
@@ -811,8 +860,8 @@ __global__ void __launch_bounds__(WGT_THREADS, 1) conv3d16_wgrad_tc_kernel(const
     const int yc = c % ych, col = c / ych;
     x0 = (col % P.tiles_x) * CV_TILE;
     z = col / P.tiles_x;
-    y0 = yc * CVR_YCH;
-    y1 = min(P.ny, y0 + CVR_YCH);
+    y0 = yc * WGT_YCH;
+    y1 = min(P.ny, y0 + WGT_YCH);
   };
   int last = -1;  // tiles this CTA handles, minus one
   for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
@@ -984,9 +1033,113 @@ __global__ void __launch_bounds__(WGT_THREADS, 1) conv3d16_wgrad_tc_kernel(const
   }
 }
 
+// =====================================================================================
+// The incoming gradient of a layer
+// =====================================================================================
+// gb = BF16(gy * (y > 0)) (gy itself without `y`) and the per-channel sums of those products in
+// FP32, in one pass: what the input and weight gradients read, and the bias gradient.  Separate
+// element-wise passes in FP32 moved six times the bytes (with them a 256^3 layer took 4.5 ms forward
+// and backward, 2.3 without; the
+// bound is HBM).  Block b sums the channels of half b mod 2; the blocks' sums are added in block
+// order in FP64, so the result does not depend on timing.
+constexpr int CGP_BLOCKS = 148 * 8, CGP_THREADS = 256;
+template <bool F32, bool MASK>
+__global__ void __launch_bounds__(CGP_THREADS) conv_grad_prep_kernel(const void* __restrict__ gy,
+                                                                     const uint4* __restrict__ y,
+                                                                     uint4* __restrict__ gb,
+                                                                     float* __restrict__ part, int nx,
+                                                                     unsigned groups)
+{
+  const int half = blockIdx.x & 1;
+  float acc[8];
+#pragma unroll
+  for (int c = 0; c < 8; c++) acc[c] = 0.0f;
+  // groups of 8 channels of one half: voxel j -> row j / nx (rows of the halves alternate)
+  for (unsigned j = (blockIdx.x >> 1) * CGP_THREADS + threadIdx.x; j < groups; j += (CGP_BLOCKS / 2) * CGP_THREADS) {
+    const unsigned row = j / (unsigned)nx;
+    const size_t o = ((size_t)row * 2 + half) * nx + (j - row * nx);
+    float g[8];
+    if constexpr (F32) {
+      const float4 a = reinterpret_cast<const float4*>(gy)[2 * o], b = reinterpret_cast<const float4*>(gy)[2 * o + 1];
+      g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w;
+      g[4] = b.x; g[5] = b.y; g[6] = b.z; g[7] = b.w;
+    } else {
+      const uint4 a = reinterpret_cast<const uint4*>(gy)[o];
+      const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        g[2 * q] = __uint_as_float(w[q] << 16);
+        g[2 * q + 1] = __uint_as_float(w[q] & 0xffff0000u);
+      }
+    }
+    if constexpr (MASK) {
+      const uint4 a = y[o];
+      const uint32_t w[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+      for (int q = 0; q < 4; q++) {  // a product, not a select: what is not finite stays so
+        g[2 * q] *= __uint_as_float(w[q] << 16) > 0.0f ? 1.0f : 0.0f;
+        g[2 * q + 1] *= __uint_as_float(w[q] & 0xffff0000u) > 0.0f ? 1.0f : 0.0f;
+      }
+    }
+    uint32_t pk[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const __nv_bfloat162 b = __floats2bfloat162_rn(g[2 * q], g[2 * q + 1]);
+      pk[q] = *reinterpret_cast<const uint32_t*>(&b);
+    }
+    gb[o] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+#pragma unroll
+    for (int c = 0; c < 8; c++) acc[c] += g[c];
+  }
+  __shared__ float sums[CGP_THREADS / 32][8];
+#pragma unroll
+  for (int c = 0; c < 8; c++) {
+    for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+    if ((threadIdx.x & 31) == 0) sums[threadIdx.x >> 5][c] = acc[c];
+  }
+  __syncthreads();
+  if (threadIdx.x < 8) {
+    float v = 0.0f;
+    for (int w = 0; w < CGP_THREADS / 32; w++) v += sums[w][threadIdx.x];
+    part[blockIdx.x * 8 + threadIdx.x] = v;
+  }
+}
+
+// db[c] = the blocks' sums of channel c; warp c of one block
+__global__ void conv_bias_sum_kernel(const float* __restrict__ part, float* __restrict__ db)
+{
+  const int c = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double v = 0.0;
+  for (int b = (c >> 3) + 2 * lane; b < CGP_BLOCKS; b += 64) v += (double)part[b * 8 + (c & 7)];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane == 0) db[c] = (float)v;
+}
+
 }  // namespace fcb
 
 using namespace fcb;
+
+extern "C" int fcb_conv3d16_grad_prep_device(const void* gy, int gyType, const void* y, void* gb, float* db,
+                                             float* scratch, int nx, int ny, int nz, void* stream)
+try {
+  if (!gy || !gb || !db || !scratch || nx <= 0 || ny <= 0 || nz <= 0 || (gyType != FCB_F32 && gyType != FCB_BF16))
+    return set_error(FCB_ERR_INVALID, "bad conv3d gradient arguments");
+  if (((uintptr_t)gy & 15) || ((uintptr_t)y & 15) || ((uintptr_t)gb & 15))
+    return set_error(FCB_ERR_INVALID, "conv3d buffers must be 16-byte aligned");
+  const long long groups = (long long)nx * ny * nz;
+  if (groups > 0x7fffffffll) return set_error(FCB_ERR_RANGE, "conv3d volume too large");
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  auto kern = gyType == FCB_F32 ? (y ? conv_grad_prep_kernel<true, true> : conv_grad_prep_kernel<true, false>)
+                                : (y ? conv_grad_prep_kernel<false, true> : conv_grad_prep_kernel<false, false>);
+  kern<<<CGP_BLOCKS, CGP_THREADS, 0, st>>>(gy, reinterpret_cast<const uint4*>(y), reinterpret_cast<uint4*>(gb), scratch,
+                                           nx, (unsigned)groups);
+  conv_bias_sum_kernel<<<1, 512, 0, st>>>(scratch, db);
+  FCB_CUDA_TRY(cudaGetLastError());
+  return ok();
+}
+FCB_CATCH_STATUS
+
+static_assert(CGP_BLOCKS * 8 == FCB_CONV_GRAD_SCRATCH, "gradient scratch");
 
 extern "C" int fcb_conv3d16_device(const void* x, const void* w, const float* bias, void* y, int yType,
                                    int nx, int ny, int nz, int relu, void* stream)
@@ -1004,13 +1157,19 @@ try {
   const bool pairs = nx % 2 == 0;
   const uint64_t dims[5] = {pairs ? 16u : 8u, (uint64_t)(pairs ? nx / 2 : nx), 2, (uint64_t)ny, (uint64_t)nz};
   const uint64_t strides[4] = {pairs ? 32u : 16u, 16ull * nx, 32ull * nx, 32ull * nx * ny};
-  const uint32_t box[5] = {pairs ? 16u : 8u, pairs ? (uint32_t)(CV_ROW + 2) / 2 : (uint32_t)CV_ROW, 1, 1, 1};
+  // FCB_CONV_SIMPLE=1: one CTA per tile; FCB_CONV_SIMPLE=2: persistent without row reuse (both for
+  // comparison, one channel half of one row per box); default: three dy taps per MMA
+  const char* env = getenv("FCB_CONV_SIMPLE");
+  const int variant = env ? atoi(env) : 0;
+  const bool simple = variant == 1 || variant == 2;
+  const uint32_t box[5] = {pairs ? 16u : 8u, pairs ? (uint32_t)(CV_ROW + 2) / 2 : (uint32_t)CV_ROW, simple ? 1u : 2u,
+                           simple ? 1u : (uint32_t)CVN_G, 1};
   FCB_TRY(encode_tmap(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(x), dims, strides, box));
   int* status = nullptr;
   FCB_TRY(device_status_ptr(&status));
   ConvParams P;
   P.pairs = pairs ? 1 : 0;
-  P.box_bytes = box[0] * box[1] * 2;
+  P.box_bytes = box[0] * box[1] * box[2] * box[3] * 2;
   P.w = reinterpret_cast<const __nv_bfloat16*>(w);
   P.bias = bias;
   P.out = y;
@@ -1021,10 +1180,6 @@ try {
   P.status = status;
   const long long tiles = (long long)P.tiles_x * ny * nz;
   if (tiles > 0x7fffffffll) return set_error(FCB_ERR_RANGE, "conv3d volume too large");
-  // FCB_CONV_SIMPLE=1: one CTA per tile; FCB_CONV_SIMPLE=2: persistent without row reuse
-  // (for comparison); default: persistent with row reuse
-  const char* env = getenv("FCB_CONV_SIMPLE");
-  const int variant = env ? atoi(env) : 0;
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1036,10 +1191,10 @@ try {
     const int grid = (int)std::min<long long>(tiles, sms);
     conv3d16p_kernel<<<grid, CVP_THREADS, CVP_SMEM, st>>>(map, P, (int)tiles);
   } else {
-    const long long nchunks = (long long)P.tiles_x * nz * ((ny + CVR_YCH - 1) / CVR_YCH);
-    FCB_CUDA_TRY(cudaFuncSetAttribute(conv3d16r_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CVR_SMEM));
+    const long long nchunks = (long long)P.tiles_x * nz * ((ny + CVN_Y - 1) / CVN_Y);
+    FCB_CUDA_TRY(cudaFuncSetAttribute(conv3d16n_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CVN_SMEM));
     const int grid = (int)std::min<long long>(nchunks, 2ll * sms);
-    conv3d16r_kernel<<<grid, CVR_THREADS, CVR_SMEM, st>>>(map, P, (int)nchunks);
+    conv3d16n_kernel<<<grid, CVN_THREADS, CVN_SMEM, st>>>(map, P, (int)nchunks);
   }
   FCB_CUDA_TRY(cudaGetLastError());
   return ok();
@@ -1074,7 +1229,7 @@ try {
     T.pairs = pairs ? 1 : 0;
     T.xbox_bytes = xbox[0] * xbox[1] * 2;
     T.status = status;
-    const long long nchunks = (long long)T.tiles_x * nz * ((ny + CVR_YCH - 1) / CVR_YCH);
+    const long long nchunks = (long long)T.tiles_x * nz * ((ny + WGT_YCH - 1) / WGT_YCH);
     if (nchunks > 0x7fffffffll) return set_error(FCB_ERR_RANGE, "conv3d volume too large");
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);

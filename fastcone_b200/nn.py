@@ -79,6 +79,22 @@ def conv3d16_wgrad(x: torch.Tensor, gy: torch.Tensor) -> torch.Tensor:
     return dw
 
 
+CONV_GRAD_SCRATCH = 9472  # FCB_CONV_GRAD_SCRATCH
+
+
+def conv3d16_grad_prep(gy: torch.Tensor, y: torch.Tensor | None):
+    """(BF16 of gy * (y > 0), its FP32 sums per channel); y None: no ReLU.  gy FP32 or BF16."""
+    _check_act(gy, "gy")
+    nz, ny, _, nx, _ = gy.shape
+    gb = torch.empty(gy.shape, device=gy.device, dtype=torch.bfloat16)
+    db = torch.empty(16, device=gy.device, dtype=torch.float32)
+    scratch = torch.empty(CONV_GRAD_SCRATCH, device=gy.device, dtype=torch.float32)
+    check(lib().fcb_conv3d16_grad_prep_device(_p(gy), _lib.FCB_F32 if gy.dtype == torch.float32 else _lib.FCB_BF16,
+                                              _p(y) if y is not None else None, _p(gb), _p(db), _p(scratch),
+                                              nx, ny, nz, _stream()))
+    return gb, db
+
+
 class Conv3d16Function(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, b, relu):
@@ -91,12 +107,19 @@ class Conv3d16Function(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gy):
         x, wk, y = ctx.saved_tensors
+        # input gradient: the same convolution with tap-flipped, transposed weights
+        wt = wk.flip(0).transpose(1, 2).contiguous()
+        if gy.dtype in (torch.float32, torch.bfloat16) and not torch.is_grad_enabled():
+            gy = gy.contiguous()
+            if gy.data_ptr() % 16 == 0:
+                gb, db = conv3d16_grad_prep(gy, y if ctx.relu else None)
+                gx = conv3d16(gb, wt, None, relu=False) if ctx.needs_input_grad[0] else None
+                dw = from_kernel_weights(conv3d16_wgrad(x, gb)) if ctx.needs_input_grad[1] else None
+                return gx, dw, db, None
         g = gy.float()
         if ctx.relu:
             g = g * (y > 0)
         gb = g.to(torch.bfloat16).contiguous()
-        # input gradient: the same convolution with tap-flipped, transposed weights
-        wt = wk.flip(0).transpose(1, 2).contiguous()
         gx = conv3d16(gb, wt, None, relu=False, out_dtype=torch.float32).to(torch.bfloat16)
         dwk = conv3d16_wgrad(x, gb)
         dw = from_kernel_weights(dwk)

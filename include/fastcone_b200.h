@@ -305,6 +305,15 @@ int fcb_conv3d16_device(const void* x, const void* w, const float* bias, void* y
 int fcb_conv3d16_wgrad_device(const void* x, const void* dy, int dyType, float* dw, int nx, int ny,
                               int nz, void* stream);
 
+/* What the gradients of a fcb_conv3d16_device layer start from: gb = BF16(gy * (y > 0)), the
+ * incoming gradient (gyType FCB_F32 / FCB_BF16) through the layer's ReLU (y: its BF16 output; NULL
+ * for a layer without one), and db[16], the FP32 sums of those products over the voxels (the bias
+ * gradient).  Same layout and alignment; scratch: FCB_CONV_GRAD_SCRATCH floats.  No counterpart in
+ * the reference. */
+#define FCB_CONV_GRAD_SCRATCH 9472
+int fcb_conv3d16_grad_prep_device(const void* gy, int gyType, const void* y, void* gb, float* db,
+                                  float* scratch, int nx, int ny, int nz, void* stream);
+
 /* Ellipsoid phantom voxelisation: vol[z][y][x] = sum of densities of ellipsoids
  * containing the voxel centre (g - volDim/2).  params: n x 16 doubles (host):
  * centre(3), semi-axes(3), row-major rotation R (9, body = R^T (p - c)), density. */
