@@ -127,7 +127,7 @@ constexpr int CV_W_BYTES = 27 * 512;          // 13824
 constexpr int CV_SMEM = CV_A_BYTES + CV_W_BYTES + 64 + 32 + 16;
 
 struct ConvParams {
-  int pairs;               // 1: boxes of voxel pairs (32-byte rows, even nx), 0: single voxels
+  int gs;                  // log2 of the voxels per box row
   uint32_t box_bytes;      // bytes of one TMA box
   const __nv_bfloat16* w;  // [27][16 out][16 in]
   const float* bias;       // [16] or null
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(128) conv3d16_kernel(const __grid_constant__ C
     for (int r = 0; r < 9; r++) {
       const int dz = r / 3, dy = r % 3;
       for (int kh = 0; kh < 2; kh++)
-        tc::tma_load_5d(A + (r * 2 + kh) * CV_RB, &xmap, &bars[0], 0, P.pairs ? (x0 >> 1) - 1 : x0 - 1, kh,
+        tc::tma_load_5d(A + (r * 2 + kh) * CV_RB, &xmap, &bars[0], 0, (x0 >> P.gs) - 1, kh,
                         y + dy - 1, z + dz - 1);
     }
   }
@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(128) conv3d16_kernel(const __grid_constant__ C
       constexpr uint32_t IDESC = tc::idesc_bf16(CV_TILE, 16);
       for (int t = 0; t < 27; t++) {
         const int r = t / 3, dx = t % 3;
-        const uint64_t ad = tc::smem_desc(abase + r * 2 * CV_RB + (dx + P.pairs) * 16, CV_RB, 128);
+        const uint64_t ad = tc::smem_desc(abase + r * 2 * CV_RB + (dx + (1 << P.gs) - 1) * 16, CV_RB, 128);
         const uint64_t bd = tc::smem_desc(wbase + t * 512, 256, 128);
         tc::mma_bf16(taddr, ad, bd, IDESC, t > 0 ? 1u : 0u);
       }
@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(CVP_THREADS, 1) conv3d16p_kernel(const __grid_
         for (int r = 0; r < 9; r++) {
           const int dz = r / 3, dy = r % 3;
           for (int kh = 0; kh < 2; kh++)
-            tc::tma_load_5d(As + (r * 2 + kh) * CV_RB, &xmap, &full[s], 0, P.pairs ? (x0 >> 1) - 1 : x0 - 1,
+            tc::tma_load_5d(As + (r * 2 + kh) * CV_RB, &xmap, &full[s], 0, (x0 >> P.gs) - 1,
                             kh, y + dy - 1, z + dz - 1);
         }
       }
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(CVP_THREADS, 1) conv3d16p_kernel(const __grid_
         const uint32_t abase = dev::smem_u32(A + s * CV_A_BYTES);
         for (int t = 0; t < 27; t++) {
           const int r = t / 3, dx = t % 3;
-          const uint64_t ad = tc::smem_desc(abase + r * 2 * CV_RB + (dx + P.pairs) * 16, CV_RB, 128);
+          const uint64_t ad = tc::smem_desc(abase + r * 2 * CV_RB + (dx + (1 << P.gs) - 1) * 16, CV_RB, 128);
           const uint64_t bd = tc::smem_desc(wbase + t * 512, 256, 128);
           tc::mma_bf16(taddr + (uint32_t)(b * 16), ad, bd, IDESC, t > 0 ? 1u : 0u);
         }
@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(CVN_THREADS, 2) conv3d16n_kernel(const __grid_
           }
           const int dz = j / groups, y = y0 - 1 + CVN_G * (j - dz * groups);
           dev::mbar_arrive_expect_tx(&full[s], P.box_bytes);
-          tc::tma_load_5d(A + s * CVN_STAGE, &xmap, &full[s], 0, P.pairs ? (x0 >> 1) - 1 : x0 - 1, 0, y, z + dz - 1);
+          tc::tma_load_5d(A + s * CVN_STAGE, &xmap, &full[s], 0, (x0 >> P.gs) - 1, 0, y, z + dz - 1);
           issued++;
           if (++s == CVN_STAGES) { s = 0; ph ^= 1u; }
         }
@@ -592,7 +592,7 @@ __global__ void __launch_bounds__(CVN_THREADS, 2) conv3d16n_kernel(const __grid_
               const int plo = max(i - 2, 0), phi = min(i, n - 1);
               const uint32_t idesc = tc::idesc_bf16(CV_TILE, 16 * (phi - plo + 1));
               const uint32_t d = taddr + (uint32_t)(16 * plo);
-              const uint32_t a0 = abase + s * CVN_STAGE + (i - i0) * 2 * half + P.pairs * 16;
+              const uint32_t a0 = abase + s * CVN_STAGE + (i - i0) * 2 * half + ((1 << P.gs) - 1) * 16;
               const uint32_t b0 = wbase + dz * 3 * CVN_WB + (plo - (i - 2)) * 256;
 #pragma unroll
               for (int dx = 0; dx < 3; dx++)
@@ -743,52 +743,61 @@ __global__ void __launch_bounds__(256) conv3d16_wgrad_kernel(const WgradParams P
 // tile (9 K-steps of 16):
 //   D_r[s*16 + co][ci] = sum_u A[s*16 + co][u] * X_r[u][ci],   A[s*16 + co][u] = dY[u + 1 - s][co]
 // with dY taken as zero outside the tile: rows s = 0, 1, 2 of D_r are the taps dx = s of row
-// r (v = u + 1 - s runs over the tile).  The three dy rows of one dz sit in consecutive
-// shared-memory slots, so one MMA per (K-step, dz) covers them: M = 128 (rows 0-47 used),
-// N = 48 (dy, ci), K = 16 -- 27 MMAs per tile give all 27 taps.  A lives in tensor memory:
-// warps 0-1 write the three shifted copies of the tile's dY (lane = s*16 + co, 16-bit voxel
-// pairs packed per 32-bit column) with tcgen05.st from the staged dY row; B is the staged X
-// rows, MN-major straight from the activation layout (8 channels of one voxel = one 16-byte
-// core-matrix row).  TMEM: 3 accumulators of 48 columns (144) + WGT_ABUF A buffers of 72.
+// r (v = u + 1 - s runs over the tile).  The nine rows (dy, dz) lie one after the other in
+// shared memory, so one MMA per K-step covers them: M = 128 (rows 0-47 used), N = 144
+// (dy, dz, ci), K = 16 -- 9 MMAs per tile give all 27 taps.  A lives in tensor memory: writer
+// warps put the three shifted copies of the tile's dY there, transposed on the way by ldmatrix
+// (dy_step); B is the staged X rows, MN-major straight from the activation layout (8 channels
+// of one voxel = one 16-byte core-matrix row).  TMEM: the accumulators' 144 columns + WGT_ABUF
+// A buffers of 72.
 // A CTA walks chunks of WGT_YCH consecutive y rows of one (x tile, z) column; each tile loads
-// its 3 new X rows into a ring of WGT_RING positions per dz, rows at positions 0 and 1 also
-// into positions WGT_RING and WGT_RING + 1, so that rows y-1, y, y+1 always occupy three
-// consecutive slots (a uniform N stride for B); dY rows are staged WGT_LEAD deep;
-//   warp 2 (one lane): TMA producer, up to WGT_LEAD tiles ahead of the MMAs;
-//   warps 0-1:         A writers (per tile), then the epilogue: TMEM lanes 0-47 of the
-//                      accumulators -> dW (FP32 atomics, once per CTA);
-//   warp 3 (one lane): MMA issuer, commits to the tile's done barrier.
+// its new X row (three planes, two halves: one box) into a ring of WGT_RING positions that runs
+// on from chunk to chunk, positions 0 and 1 also into WGT_RING and WGT_RING + 1, so that rows
+// y-1, y, y+1 always occupy three consecutive slots (a uniform N stride for B); dY rows are
+// staged WGT_LEAD deep;
+//   warp 2 (one lane):  TMA producer, up to WGT_LEAD tiles ahead of the MMAs;
+//   warps 0-1 and 4-5:  A writers, tiles in turn; then warps 0-1 the epilogue: TMEM lanes 0-47
+//                       of the accumulators -> dW (FP32 atomics, once per CTA);
+//   warp 3 (one lane):  MMA issuer, commits to the tile's done barrier.
 // Dynamic shared memory above half an SM's keeps one CTA per SM (512-column allocation).
-constexpr int WGT_THREADS = 128;
+//
+// 256^3 on one B200: 0.468 ms, the tensor pipe 70 % active (an MMA of N = 144 takes its 72 cycles;
+// 80 of the 128 rows are idle).  Before, 1.08 ms: an MMA per dz took 84 cycles at N = 48 (one per
+// K-step: 0.83), one pair of writer warps gathered dY by 16-bit loads (three pairs: 0.56;
+// ldmatrix: 0.47; ldmatrix and one pair 0.63), and every chunk began with an empty ring (0.56 to
+// 0.535).
+constexpr int WGT_GROUPS = 2;                        // pairs of A writer warps: 0-1, 4-5
+constexpr int WGT_THREADS = 192;
 constexpr int WGT_YCH = 32;                          // rows per chunk
 constexpr int WGT_KSTEPS = 9;                        // 144 voxels u per tile
-constexpr int WGT_XROW = 148;                        // staged X voxels per row (from x0 - 2)
-constexpr int WGT_RB = 2432;                         // one channel half of a staged X row, 128-B multiple
-static_assert(WGT_XROW * 16 <= WGT_RB && (WGT_KSTEPS * 16 + 1) * 16 <= WGT_XROW * 16, "X row slot");
+constexpr int WGT_XROW = 152;                        // staged X voxels per row (from x0 - group)
+constexpr int WGT_RB = WGT_XROW * 16;                // one channel half of a staged X row
+constexpr int WGT_XSLOT = 6 * WGT_RB;                // the row's three planes and two halves: one TMA box
+static_assert((WGT_KSTEPS * 16 + 7) * 16 <= WGT_RB && WGT_XROW % 8 == 0 && WGT_XSLOT % 128 == 0, "X row slot");
 constexpr int WGT_DY_BYTES = 2048;                   // one channel half of 128 dY voxels (TMA box)
 constexpr int WGT_DYH = 2432;                        // its slot: 8 zero voxels, the box, 16 zero voxels
-// Pipeline depth: X rows in a ring of WGT_RING positions per dz, so the producer runs up to
+// Pipeline depth: X rows in a ring of WGT_RING positions, so the producer runs up to
 // WGT_LEAD = WGT_RING - 2 tiles ahead of the MMAs; as many dY stages; WGT_ABUF A buffers.
 constexpr int WGT_RING = 8;
 constexpr int WGT_LEAD = WGT_RING - 2;
-constexpr int WGT_ABUF = 3;
+constexpr int WGT_ABUF = 5;
 constexpr int WGT_DY = WGT_LEAD * 2 * WGT_DYH;       // dY stages x 2 halves
 constexpr int WGT_XPOS = WGT_RING + 2;               // ring positions + the two duplicates
-constexpr int WGT_X = 3 * WGT_XPOS * 2 * WGT_RB;     // X row ring
+constexpr int WGT_X = WGT_XPOS * WGT_XSLOT;          // X row ring
 constexpr int WGT_BAR = WGT_DY + WGT_X;
 constexpr int WGT_NBAR = 2 * WGT_RING + WGT_ABUF + 1;
 constexpr int WGT_SMEM_USED = WGT_BAR + 8 * WGT_NBAR + 16;
 static_assert(WGT_DYH >= (8 + CV_TILE + 16) * 16 && WGT_DYH % 128 == 0 && WGT_DY % 128 == 0, "dY slots");
 constexpr int WGT_SMEM = 200 * 1024;                 // > half an SM: one CTA per SM
 static_assert(WGT_SMEM_USED <= WGT_SMEM, "wgrad shared memory");
-constexpr uint32_t WGT_ACOL = 144;                   // first A column (after the 9 accumulators)
+constexpr uint32_t WGT_ACOL = 144;                   // first A column (after the accumulators)
 constexpr uint32_t WGT_ACOLS = WGT_KSTEPS * 8;       // 72 columns per A buffer
 static_assert(WGT_ACOL + WGT_ABUF * WGT_ACOLS <= 512, "TMEM columns");
 
 struct WgradTcParams {
   float* dw;
-  int nx, ny, nz, tiles_x, pairs;
-  uint32_t xbox_bytes;
+  int nx, ny, nz, tiles_x;
+  int gs;  // log2 of the voxels per box row
   int* status;
 };
 
@@ -804,11 +813,17 @@ __device__ __forceinline__ void mma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
       "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// 32 lanes x 8 consecutive 32-bit columns from registers: thread i writes lane (base + i).
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8])
+// One K-step of one shift: 16 voxels x 16 channels of staged dY (16 bytes per voxel and channel
+// half) into 16 TMEM lanes (channels) x 8 columns (voxel pairs).  ldmatrix transposes: thread t
+// gets channel t / 4 and voxel pair t % 4 of each 8 x 8 matrix, as the 16x128b store wants them
+// (registers: lanes 0-7 and 8-15 of columns 0-3, then of 4-7).
+__device__ __forceinline__ void dy_step(uint32_t taddr, uint32_t row)
 {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]),
-               "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+  uint32_t r0, r1, r2, r3;
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(row) : "memory");
+  asm volatile("tcgen05.st.sync.aligned.16x128b.x2.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r0), "r"(r1), "r"(r2),
+               "r"(r3)
                : "memory");
 }
 }  // namespace tc
@@ -875,43 +890,44 @@ __global__ void __launch_bounds__(WGT_THREADS, 1) conv3d16_wgrad_tc_kernel(const
     if (lane == 0) {
       dev::tma_prefetch(&xmap);
       dev::tma_prefetch(&dymap);
-      int i = 0, issued = 0;
+      int i = 0, issued = 0, n = 0;    // tiles; rows staged
+      int pn = -WGT_RING, pi = 0;      // the previous chunk's first row and tile
       bool failed = false;
       for (int c = blockIdx.x; c < nchunks && !failed; c += gridDim.x) {
         int x0, z, y0, y1;
         chunk_of(c, x0, z, y0, y1);
+        const int cn = n, ci = i;  // this chunk's
         for (int y = y0; y < y1; y++, i++) {
-          const bool start = y == y0;
-          // the X slot refilled now (row y + 1) was last read by tile i - WGT_LEAD, every slot
-          // at a new chunk by tile i-1; the dY stage by the A writers of tile i - WGT_LEAD,
-          // which finished before its MMAs
-          const int wt = start ? i - 1 : i - WGT_LEAD;
+          const int r0 = y == y0 ? -1 : 1;  // new rows y + r0 .. y + 1
+          // The row that the last new one replaces was read last by the tile it is the first row
+          // of, or by its chunk's last tile; the dY stage by the A writers of tile i - WGT_LEAD,
+          // which finished before its MMAs.
+          const int old = n + (1 - r0) - WGT_RING;
+          const int reader = old >= cn ? ci + old - cn : old >= pn ? min(pi + old - pn, ci - 1) : pi - 1;
+          const int wt = max(reader, i - WGT_LEAD);
           if (wt >= 0 && !dev::mbar_wait(&tile_done[wt % WGT_RING], (wt / WGT_RING) & 1)) {
             dev::record_status(P.status, DEV_TIMEOUT);
             *failed_flag = 1;
             failed = true;
             break;
           }
-          const int r0 = start ? -1 : 1;  // new rows y + r0 .. y + 1
           int ncopies = 0;
-          for (int dy = r0; dy <= 1; dy++) ncopies += ((y + dy) & (WGT_RING - 1)) < 2 ? 2 : 1;
+          for (int dy = r0; dy <= 1; dy++) ncopies += ((n + dy - r0) & (WGT_RING - 1)) < 2 ? 2 : 1;
           uint64_t* full = &rows_full[i % WGT_RING];
-          dev::mbar_arrive_expect_tx(full, (uint32_t)(3 * ncopies) * 2u * P.xbox_bytes + 2u * WGT_DY_BYTES);
-          for (int dz = 0; dz < 3; dz++)
-            for (int dy = r0; dy <= 1; dy++) {
-              const int yy = y + dy, pos = yy & (WGT_RING - 1);
-              for (int dup = 0; dup < (pos < 2 ? 2 : 1); dup++) {
-                unsigned char* slot = X + (dz * WGT_XPOS + pos + dup * WGT_RING) * 2 * WGT_RB;
-                for (int kh = 0; kh < 2; kh++)
-                  tc::tma_load_5d(slot + kh * WGT_RB, &xmap, full, 0, P.pairs ? (x0 >> 1) - 1 : x0 - 1, kh, yy,
-                                  z + dz - 1);
-              }
-            }
+          dev::mbar_arrive_expect_tx(full, (uint32_t)ncopies * WGT_XSLOT + 2u * WGT_DY_BYTES);
+          for (int dy = r0; dy <= 1; dy++, n++) {
+            const int pos = n & (WGT_RING - 1);
+            for (int dup = 0; dup < (pos < 2 ? 2 : 1); dup++)
+              tc::tma_load_5d(X + (pos + dup * WGT_RING) * WGT_XSLOT, &xmap, full, 0, (x0 >> P.gs) - 1,
+                              0, y + dy, z - 1);
+          }
           unsigned char* dst = DY + (i % WGT_LEAD) * 2 * WGT_DYH + 128;  // after the 8 zero voxels
           for (int kh = 0; kh < 2; kh++)
-            tc::tma_load_5d(dst + kh * WGT_DYH, &dymap, full, 0, P.pairs ? (x0 >> 1) : x0, kh, y, z);
+            tc::tma_load_5d(dst + kh * WGT_DYH, &dymap, full, 0, x0 >> P.gs, kh, y, z);
           issued = i + 1;
         }
+        pn = cn;
+        pi = ci;
       }
       for (int j = max(0, issued - WGT_RING); j < issued; j++)
         dev::mbar_wait(&rows_full[j % WGT_RING], (j / WGT_RING) & 1, 100000000ull);
@@ -921,13 +937,13 @@ __global__ void __launch_bounds__(WGT_THREADS, 1) conv3d16_wgrad_tc_kernel(const
     if (lane == 0) {
       const uint32_t xbase = dev::smem_u32(X);
       // M = 128 (rows 0-47 used), N = 48, A K-major in TMEM, B MN-major in shared memory
-      constexpr uint32_t IDESC = tc::idesc_bf16(CV_TILE, 48) | (1u << 16);
-      int i = 0;
+      constexpr uint32_t IDESC = tc::idesc_bf16(CV_TILE, 144) | (1u << 16);
+      int i = 0, n = 0;
       bool failed = false;
       for (int c = blockIdx.x; c < nchunks && !failed; c += gridDim.x) {
         int x0, z, y0, y1;
         chunk_of(c, x0, z, y0, y1);
-        for (int y = y0; y < y1; y++, i++) {
+        for (int y = y0; y < y1; y++, i++, n++) {
           if (!dev::mbar_wait(&rows_full[i % WGT_RING], (i / WGT_RING) & 1) ||
               !dev::mbar_wait(&a_full[i % WGT_ABUF], (i / WGT_ABUF) & 1)) {
             dev::record_status(P.status, DEV_TIMEOUT);
@@ -940,38 +956,32 @@ __global__ void __launch_bounds__(WGT_THREADS, 1) conv3d16_wgrad_tc_kernel(const
           // half) every WGT_RB bytes (SBO), K core matrices of 8 voxels every 128 bytes (LBO);
           // a K-step of 16 voxels moves the start address by 256 B (16 in the descriptor's
           // address field, which stays below 2^14 inside shared memory)
-          uint64_t bd[3];
-          const int p0 = (y - 1) & (WGT_RING - 1);
-#pragma unroll
-          for (int dz = 0; dz < 3; dz++)
-            bd[dz] = tc::smem_desc(xbase + (dz * WGT_XPOS + p0) * 2 * WGT_RB + P.pairs * 16, 128, WGT_RB);
+          const uint64_t bd = tc::smem_desc(xbase + (n & (WGT_RING - 1)) * WGT_XSLOT + ((1 << P.gs) - 1) * 16, 128, WGT_RB);
           const uint32_t aaddr = taddr + WGT_ACOL + (uint32_t)(i % WGT_ABUF) * WGT_ACOLS;
-          for (int ks = 0; ks < WGT_KSTEPS; ks++) {
-            const uint32_t acc = (i > 0 || ks > 0) ? 1u : 0u;
-#pragma unroll
-            for (int dz = 0; dz < 3; dz++)
-              tc::mma_bf16_ts(taddr + (uint32_t)(dz * 48), aaddr + (uint32_t)(ks * 8), bd[dz] + (uint64_t)(ks * 16),
-                              IDESC, acc);
-          }
+          for (int ks = 0; ks < WGT_KSTEPS; ks++)
+            tc::mma_bf16_ts(taddr, aaddr + (uint32_t)(ks * 8), bd + (uint64_t)(ks * 16), IDESC, i > 0 || ks > 0);
           tc::mma_commit(&tile_done[i % WGT_RING]);
         }
+        n += 2;  // the chunk's last two rows
       }
       // one phase that completes when every MMA issued here has (or at once if none was)
       if (i > 0) tc::mma_commit(fin);
       else dev::mbar_arrive(fin);
     }
-  } else {
-    // ---------------------------------------------------------------- A writers (warps 0-1)
-    const int m = warp * 32 + lane;  // TMEM lane = s * 16 + co
-    const int s = m >> 4, co = m & 15;
-    const int se = s < 3 ? s : 2;    // lanes 48-63 (unused rows of D) copy s = 2
-    const uint32_t lane_base = (uint32_t)(warp * 32) << 16;
+  } else if ((warp & 3) < 2) {
+    // ---------------------------------------------------------------- A writers (warps 0-1, 4-5, ..)
+    const int group = warp >> 2;
+    const int s0 = 2 * (warp & 1);  // first of the shifts s = 0, 1 or s = 2 (TMEM lanes 16 s + co)
+    const uint32_t lane_base = (uint32_t)(16 * s0) << 16;
+    // this lane's row of the four 8 x 8 matrices (voxel half, channel half) of a K-step
+    const uint32_t row = dev::smem_u32(DY) + (lane >> 3 & 1) * WGT_DYH + (8 + (lane >> 4) * 8 + (lane & 7)) * 16;
     int i = 0;
     bool failed = false;
     for (int c = blockIdx.x; c < nchunks && !failed; c += gridDim.x) {
       int x0, z, y0, y1;
       chunk_of(c, x0, z, y0, y1);
       for (int y = y0; y < y1; y++, i++) {
+        if (i % WGT_GROUPS != group) continue;
         // the dY row of tile i is staged, and the A buffer's previous readers (the MMAs of
         // tile i - WGT_ABUF) are done
         bool ok = dev::mbar_wait(&rows_full[i % WGT_RING], (i / WGT_RING) & 1);
@@ -987,16 +997,12 @@ __global__ void __launch_bounds__(WGT_THREADS, 1) conv3d16_wgrad_tc_kernel(const
         }
         tc::fence_after();
         // A[u] = dY[x0 + rel], rel = 16 ks + k - s: slot voxel rel + 8 (zero outside the tile)
-        const unsigned short* dyb = reinterpret_cast<const unsigned short*>(
-            DY + (i % WGT_LEAD) * 2 * WGT_DYH + (co >> 3) * WGT_DYH + (8 - se) * 16) + (co & 7);
-        const uint32_t acol = WGT_ACOL + (uint32_t)(i % WGT_ABUF) * WGT_ACOLS;
-#pragma unroll 1
-        for (int ks = 0; ks < WGT_KSTEPS; ks++) {
-          const unsigned short* p = dyb + ks * 16 * 8;
-          uint32_t pk[8];
+        const uint32_t src = row + (uint32_t)(i % WGT_LEAD) * 2 * WGT_DYH;
+        const uint32_t dst = taddr + lane_base + WGT_ACOL + (uint32_t)(i % WGT_ABUF) * WGT_ACOLS;
 #pragma unroll
-          for (int j = 0; j < 8; j++) pk[j] = (uint32_t)p[(2 * j) * 8] | ((uint32_t)p[(2 * j + 1) * 8] << 16);
-          tc::tmem_st8(taddr + lane_base + acol + (uint32_t)(ks * 8), pk);
+        for (int ks = 0; ks < WGT_KSTEPS; ks++) {
+          tc::dy_step(dst + (uint32_t)(ks * 8), src + (uint32_t)(ks * 256 - s0 * 16));
+          if (s0 == 0) tc::dy_step(dst + (16u << 16) + (uint32_t)(ks * 8), src + (uint32_t)(ks * 256 - 16));
         }
         tc::tmem_wait_st();
         tc::fence_before();
@@ -1005,15 +1011,16 @@ __global__ void __launch_bounds__(WGT_THREADS, 1) conv3d16_wgrad_tc_kernel(const
       }
     }
     // ---------------------------------------------------------------- epilogue
-    if (last >= 0) {
+    if (last >= 0 && group == 0) {
+      const int s = 2 * warp + (lane >> 4), co = lane & 15;
       const bool done = __all_sync(0xffffffffu, dev::mbar_wait(fin, 0)) != 0;
       tc::fence_after();
       if (done && !*failed_flag) {
         for (int r = 0; r < 9; r++) {
           uint32_t v[16];
-          tc::tmem_ld16(taddr + lane_base + (uint32_t)(r * 16), v);
+          tc::tmem_ld16(taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)(r * 16), v);
           if (s < 3) {
-            float* d = P.dw + ((r * 3 + s) * 16 + co) * 16;
+            float* d = P.dw + (((r % 3 * 3 + r / 3) * 3 + s) * 16 + co) * 16;  // columns (dy, dz), taps (dz, dy, dx)
 #pragma unroll
             for (int q = 0; q < 16; q++) atomicAdd(d + q, __uint_as_float(v[q]));
           }
@@ -1038,9 +1045,8 @@ __global__ void __launch_bounds__(WGT_THREADS, 1) conv3d16_wgrad_tc_kernel(const
 // =====================================================================================
 // gb = BF16(gy * (y > 0)) (gy itself without `y`) and the per-channel sums of those products in
 // FP32, in one pass: what the input and weight gradients read, and the bias gradient.  Separate
-// element-wise passes in FP32 moved six times the bytes (with them a 256^3 layer took 4.5 ms forward
-// and backward, 2.3 without; the
-// bound is HBM).  Block b sums the channels of half b mod 2; the blocks' sums are added in block
+// element-wise passes in FP32 moved six times the bytes (and took 2.2 ms more of a 256^3 layer's
+// forward and backward); the bound is HBM.  Block b sums the channels of half b mod 2; the blocks' sums are added in block
 // order in FP64, so the result does not depend on timing.
 constexpr int CGP_BLOCKS = 148 * 8, CGP_THREADS = 256;
 template <bool F32, bool MASK>
@@ -1141,6 +1147,19 @@ FCB_CATCH_STATUS
 
 static_assert(CGP_BLOCKS * 8 == FCB_CONV_GRAD_SCRATCH, "gradient scratch");
 
+// log2 of the voxels per TMA box row.  Activations are [z][y][2][x][8], a row of one channel half
+// contiguous, read as dims (channels of 2^gs voxels, x >> gs, half, y, z): the copy engine takes a
+// box row at a time, and rows of 16 bytes fetch every sector twice.  A tile's box starts one group
+// before its first voxel, its operands 2^gs - 1 voxels into the box, so gs <= `most` must divide nx.
+// The weight gradient takes groups of up to 8 (256^3: 0.468 ms, with pairs 0.49); the forward
+// kernel, not bound by its copies, pairs (groups of 8: 0.444 ms, with pairs 0.440).
+static int box_group(int nx, int most)
+{
+  int gs = most;
+  while (nx & ((1 << gs) - 1)) gs--;
+  return gs;
+}
+
 extern "C" int fcb_conv3d16_device(const void* x, const void* w, const float* bias, void* y, int yType,
                                    int nx, int ny, int nz, int relu, void* stream)
 try {
@@ -1150,25 +1169,21 @@ try {
     return set_error(FCB_ERR_INVALID, "conv3d buffers must be 16-byte aligned");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   CUtensorMap map;
-  // [z][y][2][x][8]: dims (channels of a voxel pair or of one voxel, x, half, y, z).  With
-  // even nx a box row is a voxel pair (32 bytes, one L2 sector): 66 pairs cover voxels
-  // x0-2 .. x0+129, and the MMA operands start one voxel into the box.  Single-voxel rows
-  // (16 bytes) would fetch every sector twice.
-  const bool pairs = nx % 2 == 0;
-  const uint64_t dims[5] = {pairs ? 16u : 8u, (uint64_t)(pairs ? nx / 2 : nx), 2, (uint64_t)ny, (uint64_t)nz};
-  const uint64_t strides[4] = {pairs ? 32u : 16u, 16ull * nx, 32ull * nx, 32ull * nx * ny};
   // FCB_CONV_SIMPLE=1: one CTA per tile; FCB_CONV_SIMPLE=2: persistent without row reuse (both for
   // comparison, one channel half of one row per box); default: three dy taps per MMA
   const char* env = getenv("FCB_CONV_SIMPLE");
   const int variant = env ? atoi(env) : 0;
   const bool simple = variant == 1 || variant == 2;
-  const uint32_t box[5] = {pairs ? 16u : 8u, pairs ? (uint32_t)(CV_ROW + 2) / 2 : (uint32_t)CV_ROW, simple ? 1u : 2u,
+  const int gs = box_group(nx, 1), group = 1 << gs;
+  const uint64_t dims[5] = {8ull * group, (uint64_t)(nx / group), 2, (uint64_t)ny, (uint64_t)nz};
+  const uint64_t strides[4] = {16ull * group, 16ull * nx, 32ull * nx, 32ull * nx * ny};
+  const uint32_t box[5] = {8u * group, (uint32_t)((CV_ROW + 2 * group - 2) / group), simple ? 1u : 2u,
                            simple ? 1u : (uint32_t)CVN_G, 1};
   FCB_TRY(encode_tmap(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(x), dims, strides, box));
   int* status = nullptr;
   FCB_TRY(device_status_ptr(&status));
   ConvParams P;
-  P.pairs = pairs ? 1 : 0;
+  P.gs = gs;
   P.box_bytes = box[0] * box[1] * box[2] * box[3] * 2;
   P.w = reinterpret_cast<const __nv_bfloat16*>(w);
   P.bias = bias;
@@ -1212,11 +1227,11 @@ try {
   if (dyType == FCB_BF16 && !(simt && simt[0] == '1')) {
     if (((uintptr_t)x & 15) || ((uintptr_t)dy & 15))
       return set_error(FCB_ERR_INVALID, "conv3d wgrad buffers must be 16-byte aligned");
-    const bool pairs = nx % 2 == 0;
-    const uint64_t dims[5] = {pairs ? 16u : 8u, (uint64_t)(pairs ? nx / 2 : nx), 2, (uint64_t)ny, (uint64_t)nz};
-    const uint64_t strides[4] = {pairs ? 32u : 16u, 16ull * nx, 32ull * nx, 32ull * nx * ny};
-    const uint32_t xbox[5] = {pairs ? 16u : 8u, pairs ? (uint32_t)WGT_XROW / 2 : (uint32_t)WGT_XROW - 2, 1, 1, 1};
-    const uint32_t dybox[5] = {pairs ? 16u : 8u, pairs ? (uint32_t)CV_TILE / 2 : (uint32_t)CV_TILE, 1, 1, 1};
+    const int gs = box_group(nx, 3), group = 1 << gs;
+    const uint64_t dims[5] = {8ull * group, (uint64_t)(nx / group), 2, (uint64_t)ny, (uint64_t)nz};
+    const uint64_t strides[4] = {16ull * group, 16ull * nx, 32ull * nx, 32ull * nx * ny};
+    const uint32_t xbox[5] = {8u * group, (uint32_t)(WGT_XROW / group), 2, 1, 3};
+    const uint32_t dybox[5] = {8u * group, (uint32_t)(CV_TILE / group), 1, 1, 1};
     CUtensorMap xmap, dymap;
     FCB_TRY(encode_tmap(&xmap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(x), dims, strides, xbox));
     FCB_TRY(encode_tmap(&dymap, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(dy), dims, strides, dybox));
@@ -1226,8 +1241,7 @@ try {
     T.dw = dw;
     T.nx = nx; T.ny = ny; T.nz = nz;
     T.tiles_x = (nx + CV_TILE - 1) / CV_TILE;
-    T.pairs = pairs ? 1 : 0;
-    T.xbox_bytes = xbox[0] * xbox[1] * 2;
+    T.gs = gs;
     T.status = status;
     const long long nchunks = (long long)T.tiles_x * nz * ((ny + WGT_YCH - 1) / WGT_YCH);
     if (nchunks > 0x7fffffffll) return set_error(FCB_ERR_RANGE, "conv3d volume too large");
