@@ -128,6 +128,7 @@ constexpr int CV_SMEM = CV_A_BYTES + CV_W_BYTES + 64 + 32 + 16;
 
 struct ConvParams {
   int gs;                  // log2 of the voxels per box row
+  int yl, zl;              // rows and planes of a walk (conv3d16n_kernel)
   uint32_t box_bytes;      // bytes of one TMA box
   const __nv_bfloat16* w;  // [27][16 out][16 in]
   const float* bias;       // [16] or null
@@ -435,46 +436,47 @@ __global__ void __launch_bounds__(CVP_THREADS, 1) conv3d16p_kernel(const __grid_
 
 // The default form.  An MMA of N = 16 reads its 4 KB of A from shared memory for 8 cycles' worth of
 // arithmetic, so the kernels above are bound by operand reads and a fixed cost per MMA (27 per tile
-// at about 53 cycles).  Here one MMA covers the three dy taps: an input row contributes to the
-// output rows above, at and below it, whose accumulators lie side by side in tensor memory, so one
-// A row (per dz and dx) times the three taps' weights (N = 48) updates all three.  Nine MMAs per
-// row instead of 27, and every staged row is used once.
-// A CTA walks chunks of up to CVN_Y output rows of one (x tile, z) column, dz by dz, so that every
-// output gathers its taps in the order dz, dy, dx of the kernels above: the same bits (and the same
-// signs around zero, which a ReLU's gradient passes on).  Output row p of a chunk owns TMEM columns
-// 16 p .. 16 p + 15.  Input row i (y0 - 1 + i) updates rows i - 2, i - 1, i of those the chunk has;
-// with dz = 2 it completes row i - 2.
-//   warp 4 (one lane): TMA producer, CVN_G consecutive input rows per stage, one box each (a wait
-//                      and a commit per row cost as much as the row's MMAs: 0.500 ms);
+// at about 53 cycles).  Here one MMA covers the three dz taps: an input plane contributes to the
+// output planes below, at and above it, whose accumulators lie side by side in tensor memory, so one
+// A row (per dy and dx) times the three taps' weights (N = 48) updates all three.
+// A CTA walks up to P.zl output planes of CVN_Y rows of one x tile.  Output plane q of the walk has
+// the columns of block q mod 3 of its row, so the order of the taps along N turns with the plane:
+// the weights lie as dz = 2, 1, 0, 2, 1, of which each order is a window.  Input plane k updates
+// planes k - 1, k, k + 1 of those the walk has and completes plane k - 1; the planes of a row are
+// updated by nine MMAs in a row, and every output gathers its taps in the order dz, dy, dx of the
+// kernels above: the same bits (and the same signs around zero, which a ReLU's gradient passes on).
+//   warp 4 (one lane): TMA producer, the CVN_Y + 2 rows of an input plane per stage, one box;
 //   warp 5 (one lane): MMA issuer; commits free the stage and hand finished rows over;
 //   warps 0-3:         epilogue: read their TMEM lane quadrant of a finished row, clear it for the
-//                      next chunk (accumulators start from zero: rows join at different MMAs),
-//                      release it, then bias / ReLU / store.
-// 256^3 on one B200: 0.442 ms per layer, 0.646 with N = 16 and row reuse (HBM floor 0.165).  The
-// operand reads of an MMA take 44 cycles of shared memory; here one takes 97, since three MMAs on
-// one accumulator are followed by three on one that overlaps it (with nine in a row, the taps in
-// another order, 0.318).  Twice as many epilogue warps changed nothing.
-constexpr int CVN_Y = 16;
-constexpr int CVN_G = 3;                   // input rows per stage
-constexpr int CVN_STAGES = 5;
+//                      plane that takes its block next (accumulators start from zero), release it,
+//                      then bias / ReLU / store.
+// 256^3 on one B200: 0.328 ms per layer (HBM floor 0.165; the operand reads of an MMA take 44 cycles
+// of shared memory, here one takes about 65).  0.646 with N = 16 and row reuse; 0.440 with N = 48
+// over the dy taps of one plane, where three MMAs on one accumulator were followed by three on one
+// that overlapped it (97 cycles each) and a plane was staged three times.
+constexpr int CVN_Y = 5;                   // output rows of a walk
+constexpr int CVN_STAGES = 3;
 constexpr int CVN_THREADS = 192;
-constexpr int CVN_STAGE = CVN_G * 2 * (CV_ROW + 2) * 16;  // [row][channel half][voxel] x 16 B
-constexpr int CVN_WB = 48 * 32;            // weights of one (dz, dx): [K half][dy = 2, 1, 0][16 out] x 16 B
-constexpr int CVN_COLS = 16 * CVN_Y;       // TMEM columns: two CTAs per SM
-constexpr int CVN_SMEM = CVN_STAGES * CVN_STAGE + 9 * CVN_WB + 64 + 8 * (2 * CVN_STAGES + 2 * CVN_Y) + 16;
-static_assert(CVN_STAGE % 128 == 0 && 3 * CVN_SMEM > 227 * 1024 && 2 * CVN_SMEM < 225 * 1024 && 2 * CVN_COLS <= 512,
+constexpr int CVN_STAGE = (CVN_Y + 2) * 2 * (CV_ROW + 2) * 16;  // [row][channel half][voxel] x 16 B
+constexpr int CVN_WB = 80 * 32;            // weights of one (dy, dx): [K half][dz = 2, 1, 0, 2, 1][16 out] x 16 B
+constexpr int CVN_COLS = 256;              // TMEM columns (48 a row): two CTAs per SM
+constexpr int CVN_ACC = 3 * CVN_Y;         // accumulator blocks
+constexpr int CVN_SMEM = CVN_STAGES * CVN_STAGE + 9 * CVN_WB + 64 + 8 * (2 * CVN_STAGES + 2 * CVN_ACC) + 16;
+static_assert(CVN_STAGE % 128 == 0 && 3 * CVN_SMEM > 227 * 1024 && 2 * (CVN_SMEM + 1024) <= 228 * 1024 &&
+                  16 * CVN_ACC <= CVN_COLS && 2 * CVN_COLS <= 512,
               "two CTAs per SM");
 
-// The chunks of a volume: c -> x tile, z, rows [y0, y1)
+// The walks of a volume: c -> x tile, rows [y0, y1), planes [z0, z1)
 struct ConvChunks {
-  int tiles_x, ny, ych;
-  __device__ __forceinline__ void at(int c, int& x0, int& z, int& y0, int& y1) const
+  int tiles_x, ny, nz, yl, zl, ych;
+  __device__ __forceinline__ void at(int c, int& x0, int& y0, int& y1, int& z0, int& z1) const
   {
     const int yc = c % ych, col = c / ych;
     x0 = (col % tiles_x) * CV_TILE;
-    z = col / tiles_x;
-    y0 = yc * CVN_Y;
-    y1 = min(ny, y0 + CVN_Y);
+    y0 = yc * yl;
+    y1 = min(ny, y0 + yl);
+    z0 = col / tiles_x * zl;
+    z1 = min(nz, z0 + zl);
   }
 };
 
@@ -488,21 +490,21 @@ __global__ void __launch_bounds__(CVN_THREADS, 2) conv3d16n_kernel(const __grid_
   float* bias = reinterpret_cast<float*>(Wsm + 9 * CVN_WB);
   uint64_t* full = reinterpret_cast<uint64_t*>(Wsm + 9 * CVN_WB + 64);
   uint64_t* empty = full + CVN_STAGES;
-  uint64_t* accf = empty + CVN_STAGES;  // [CVN_Y] output row complete (MMA commit)
-  uint64_t* acce = accf + CVN_Y;        // [CVN_Y] output row read and cleared (4 epilogue warps)
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(acce + CVN_Y);
+  uint64_t* accf = empty + CVN_STAGES;  // [CVN_ACC] row of a plane complete (MMA commit)
+  uint64_t* acce = accf + CVN_ACC;      // [CVN_ACC] row read and cleared (4 epilogue warps)
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(acce + CVN_ACC);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const ConvChunks CH{P.tiles_x, P.ny, (P.ny + CVN_Y - 1) / CVN_Y};
+  const ConvChunks CH{P.tiles_x, P.ny, P.nz, P.yl, P.zl, (P.ny + P.yl - 1) / P.yl};
 
   if (threadIdx.x == 0) {
     for (int q = 0; q < CVN_STAGES; q++) {
       dev::mbar_init(&full[q], 1);
       dev::mbar_init(&empty[q], 1);
     }
-    for (int p = 0; p < CVN_Y; p++) {
-      dev::mbar_init(&accf[p], 1);
-      dev::mbar_init(&acce[p], 4);
+    for (int q = 0; q < CVN_ACC; q++) {
+      dev::mbar_init(&accf[q], 1);
+      dev::mbar_init(&acce[q], 4);
     }
     dev::fence_mbar_init();
   }
@@ -510,13 +512,13 @@ __global__ void __launch_bounds__(CVN_THREADS, 2) conv3d16n_kernel(const __grid_
     tc::tmem_alloc(tslot, CVN_COLS);
     tc::tmem_relinquish();
   }
-  // weights: (dz, dx), K half kh, dy block (2, 1, 0), out channel n: 16 bytes of 8 in-channels
+  // weights: (dy, dx), K half kh, dz block, out channel n: 16 bytes of 8 in-channels
   const uint4* wg = reinterpret_cast<const uint4*>(P.w);
-  for (int i = threadIdx.x; i < 27 * 16 * 2; i += blockDim.x) {
-    const int t = i / 32, n = (i / 2) % 16, kh = i % 2;
-    const int dz = t / 9, dy = (t / 3) % 3, dx = t % 3;
-    reinterpret_cast<uint4*>(Wsm + (dz * 3 + dx) * CVN_WB + kh * (CVN_WB / 2) + ((2 - dy) * 16 + n) * 16)[0] =
-        wg[(t * 16 + n) * 2 + kh];
+  for (int i = threadIdx.x; i < 45 * 16 * 2; i += blockDim.x) {
+    const int t = i / 160, blk = i / 32 % 5, n = i / 2 % 16, kh = i % 2;
+    const int dz = (5 - blk) % 3;  // 2, 1, 0, 2, 1
+    reinterpret_cast<uint4*>(Wsm + t * CVN_WB + kh * (CVN_WB / 2) + (blk * 16 + n) * 16)[0] =
+        wg[((dz * 9 + t) * 16 + n) * 2 + kh];
   }
   if (threadIdx.x < 16) bias[threadIdx.x] = P.bias ? P.bias[threadIdx.x] : 0.0f;
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -526,7 +528,7 @@ __global__ void __launch_bounds__(CVN_THREADS, 2) conv3d16n_kernel(const __grid_
   const uint32_t taddr = *tslot;
   const uint32_t lanes = (uint32_t)(warp * 32) << 16;
   if (warp < 4) {
-    for (int p = 0; p < CVN_Y; p++) tc::tmem_zero16(taddr + lanes + (uint32_t)(16 * p));
+    for (int q = 0; q < CVN_ACC; q++) tc::tmem_zero16(taddr + lanes + (uint32_t)(16 * q));
     tc::tmem_wait_st();
   }
   tc::fence_before();
@@ -541,18 +543,16 @@ __global__ void __launch_bounds__(CVN_THREADS, 2) conv3d16n_kernel(const __grid_
       uint32_t ph = 0;
       bool failed = false;
       for (int c = blockIdx.x; c < nchunks && !failed; c += gridDim.x) {
-        int x0, z, y0, y1;
-        CH.at(c, x0, z, y0, y1);
-        const int groups = (y1 - y0 + 2 + CVN_G - 1) / CVN_G;
-        for (int j = 0; j < 3 * groups; j++) {  // dz slowest; rows past the chunk's are read, not used
+        int x0, y0, y1, z0, z1;
+        CH.at(c, x0, y0, y1, z0, z1);
+        for (int z = z0 - 1; z <= z1; z++) {  // rows past the walk's are read, not used
           if (issued >= CVN_STAGES && !dev::mbar_wait(&empty[s], ph ^ 1u)) {
             dev::record_status(P.status, DEV_TIMEOUT);
             failed = true;
             break;
           }
-          const int dz = j / groups, y = y0 - 1 + CVN_G * (j - dz * groups);
           dev::mbar_arrive_expect_tx(&full[s], P.box_bytes);
-          tc::tma_load_5d(A + s * CVN_STAGE, &xmap, &full[s], 0, (x0 >> P.gs) - 1, 0, y, z + dz - 1);
+          tc::tma_load_5d(A + s * CVN_STAGE, &xmap, &full[s], 0, (x0 >> P.gs) - 1, 0, y0 - 1, z);
           issued++;
           if (++s == CVN_STAGES) { s = 0; ph ^= 1u; }
         }
@@ -567,44 +567,59 @@ __global__ void __launch_bounds__(CVN_THREADS, 2) conv3d16n_kernel(const __grid_
       const uint32_t wbase = dev::smem_u32(Wsm), abase = dev::smem_u32(A);
       int s = 0;
       uint32_t ph = 0;
-      uint32_t used = 0;  // bit p: parity of the uses of output row p so far
+      uint32_t used = 0;  // bit q: parity of the uses of accumulator block q so far
       int stages = 0;     // stages issued
-      const uint32_t half = P.box_bytes / (2 * CVN_G);  // one channel half of one staged row
+      const uint32_t half = P.box_bytes / (2 * (CVN_Y + 2));  // one channel half of one staged row
       bool failed = false;
       for (int c = blockIdx.x; c < nchunks && !failed; c += gridDim.x) {
-        int x0, z, y0, y1;
-        CH.at(c, x0, z, y0, y1);
-        const int n = y1 - y0;
-        for (int dz = 0; dz < 3 && !failed; dz++)
-          for (int i0 = 0; i0 < n + 2; i0 += CVN_G) {
-            const int i1 = min(i0 + CVN_G, n + 2);
-            bool ok = dev::mbar_wait(&full[s], ph);
-            // with dz = 0 the chunk's rows join: their previous uses must have been read and cleared
-            if (dz == 0)
-              for (int i = i0; ok && i < min(i1, n); i++) ok = dev::mbar_wait(&acce[i], ((used >> i) & 1u) ^ 1u);
-            if (!ok) {
-              dev::record_status(P.status, DEV_TIMEOUT);
-              failed = true;
-              break;
+        int x0, y0, y1, z0, z1;
+        CH.at(c, x0, y0, y1, z0, z1);
+        const int n = y1 - y0, len = z1 - z0;
+        int b1 = 0;  // block of plane k + 1
+        for (int k = -1; k <= len; k++) {
+          bool ok = dev::mbar_wait(&full[s], ph);
+          const int b0 = b1 == 0 ? 2 : b1 - 1, bm = b1 == 2 ? 0 : b1 + 1;  // of planes k, k - 1
+          tc::fence_after();
+          for (int p = 0; ok && p < n; p++) {
+            if (k + 1 < len) {  // plane k + 1 joins: the block's previous plane must have been read and cleared
+              const int q = 3 * p + b1;
+              ok = dev::mbar_wait(&acce[q], ((used >> q) & 1u) ^ 1u);
+              if (!ok) break;
+              used ^= 1u << q;
+              tc::fence_after();
             }
-            tc::fence_after();
-            for (int i = i0; i < i1; i++) {
-              const int plo = max(i - 2, 0), phi = min(i, n - 1);
-              const uint32_t idesc = tc::idesc_bf16(CV_TILE, 16 * (phi - plo + 1));
-              const uint32_t d = taddr + (uint32_t)(16 * plo);
-              const uint32_t a0 = abase + s * CVN_STAGE + (i - i0) * 2 * half + ((1 << P.gs) - 1) * 16;
-              const uint32_t b0 = wbase + dz * 3 * CVN_WB + (plo - (i - 2)) * 256;
+            const uint32_t d = taddr + (uint32_t)(48 * p);
+            const uint32_t a0 = abase + s * CVN_STAGE + p * 2 * half + ((1 << P.gs) - 1) * 16;
+            // blocks [col, col + count), weights from block `win` of 2, 1, 0, 2, 1
+            auto mmas = [&](int col, int count, int win) {
+              const uint32_t idesc = tc::idesc_bf16(CV_TILE, 16 * count);
+              const uint32_t w0 = wbase + win * 256;
 #pragma unroll
-              for (int dx = 0; dx < 3; dx++)
-                tc::mma_bf16(d, tc::smem_desc(a0 + dx * 16, half, 128),
-                             tc::smem_desc(b0 + dx * CVN_WB, CVN_WB / 2, 128), idesc, 1u);
-              if (dz == 2 && i >= 2) tc::mma_commit(&accf[i - 2]);
+              for (int t = 0; t < 9; t++)
+                tc::mma_bf16(d + 16 * col, tc::smem_desc(a0 + (t / 3) * 2 * half + (t % 3) * 16, half, 128),
+                             tc::smem_desc(w0 + t * CVN_WB, CVN_WB / 2, 128), idesc, 1u);
+            };
+            const bool vm = k >= 1, v0 = k >= 0 && k < len, v1 = k + 1 < len;  // planes k - 1, k, k + 1 of the walk
+            if (vm && v0 && v1) mmas(0, 3, bm == 0 ? 0 : bm == 1 ? 2 : 1);
+            else if (v0 && v1 && b0 < b1) mmas(b0, 2, 1);
+            else if (vm && v0 && bm < b0) mmas(bm, 2, 0);
+            else {
+              if (vm) mmas(bm, 1, 0);
+              if (v0) mmas(b0, 1, 1);
+              if (v1) mmas(b1, 1, 2);
             }
-            tc::mma_commit(&empty[s]);
-            stages++;
-            if (++s == CVN_STAGES) { s = 0; ph ^= 1u; }
+            if (vm) tc::mma_commit(&accf[3 * p + bm]);
           }
-        if (!failed) used ^= (1u << n) - 1u;
+          if (!ok) {
+            dev::record_status(P.status, DEV_TIMEOUT);
+            failed = true;
+            break;
+          }
+          b1 = b1 == 2 ? 0 : b1 + 1;
+          tc::mma_commit(&empty[s]);
+          stages++;
+          if (++s == CVN_STAGES) { s = 0; ph ^= 1u; }
+        }
       }
       // every MMA issued must be complete before the columns are released: the last stage's commit
       if (stages > 0) dev::mbar_wait(&empty[(stages - 1) % CVN_STAGES], ((stages - 1) / CVN_STAGES) & 1, 100000000ull);
@@ -614,25 +629,27 @@ __global__ void __launch_bounds__(CVN_THREADS, 2) conv3d16n_kernel(const __grid_
     uint32_t used = 0;
     bool failed = false;
     for (int c = blockIdx.x; c < nchunks && !failed; c += gridDim.x) {
-      int x0, z, y0, y1;
-      CH.at(c, x0, z, y0, y1);
+      int x0, y0, y1, z0, z1;
+      CH.at(c, x0, y0, y1, z0, z1);
       const int n = y1 - y0;
       const int xv = x0 + warp * 32 + lane;
-      for (int p = 0; p < n; p++) {
+      for (int i = 0; i < n * (z1 - z0); i++) {
+        const int k = i / n, p = i - k * n, z = z0 + k, q = 3 * p + k % 3;
         // warp-uniform: the tcgen05 instructions below are warp-collective
-        if (!__all_sync(0xffffffffu, dev::mbar_wait(&accf[p], (used >> p) & 1u))) {
+        if (!__all_sync(0xffffffffu, dev::mbar_wait(&accf[q], (used >> q) & 1u))) {
           if (lane == 0) dev::record_status(P.status, DEV_TIMEOUT);
           failed = true;
           break;
         }
+        used ^= 1u << q;
         tc::fence_after();
         uint32_t r[16];
-        tc::tmem_ld16(taddr + lanes + (uint32_t)(16 * p), r);
-        tc::tmem_zero16(taddr + lanes + (uint32_t)(16 * p));
+        tc::tmem_ld16(taddr + lanes + (uint32_t)(16 * q), r);
+        tc::tmem_zero16(taddr + lanes + (uint32_t)(16 * q));
         tc::tmem_wait_st();
         tc::fence_before();
         __syncwarp();
-        if (lane == 0) dev::mbar_arrive(&acce[p]);
+        if (lane == 0) dev::mbar_arrive(&acce[q]);
         if (xv < P.nx) {
           const int y = y0 + p;
           float v[16];
@@ -662,7 +679,6 @@ __global__ void __launch_bounds__(CVN_THREADS, 2) conv3d16n_kernel(const __grid_
           }
         }
       }
-      used ^= (1u << n) - 1u;
     }
   }
   tc::fence_before();
@@ -1178,7 +1194,7 @@ try {
   const uint64_t dims[5] = {8ull * group, (uint64_t)(nx / group), 2, (uint64_t)ny, (uint64_t)nz};
   const uint64_t strides[4] = {16ull * group, 16ull * nx, 32ull * nx, 32ull * nx * ny};
   const uint32_t box[5] = {8u * group, (uint32_t)((CV_ROW + 2 * group - 2) / group), simple ? 1u : 2u,
-                           simple ? 1u : (uint32_t)CVN_G, 1};
+                           simple ? 1u : (uint32_t)(CVN_Y + 2), 1};
   FCB_TRY(encode_tmap(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void*>(x), dims, strides, box));
   int* status = nullptr;
   FCB_TRY(device_status_ptr(&status));
@@ -1206,7 +1222,25 @@ try {
     const int grid = (int)std::min<long long>(tiles, sms);
     conv3d16p_kernel<<<grid, CVP_THREADS, CVP_SMEM, st>>>(map, P, (int)tiles);
   } else {
-    const long long nchunks = (long long)P.tiles_x * nz * ((ny + CVN_Y - 1) / CVN_Y);
+    // Rows and planes per walk: those with the least work on the busiest CTA, (planes + 2) passes over
+    // the rows per walk and about one row's worth to start each pass; three rows at least (fewer
+    // would wait for the epilogue).  64^3: 3 x 5, 22.3 us (5 x 3: 24.6); 256^3: 5 x 32.
+    long long nchunks = 0, best = 0;
+    for (int yl = std::min(3, ny); yl <= std::min(CVN_Y, ny); yl++) {
+      const long long cols = (long long)P.tiles_x * ((ny + yl - 1) / yl);
+      const int least = (nz + 63) / 64, most = std::min(nz, least + 2 * sms);
+      for (int walks = least; walks <= most; walks++) {
+        const int zl = (nz + walks - 1) / walks;
+        const long long units = cols * ((nz + zl - 1) / zl);
+        const long long cost = (units + 2 * sms - 1) / (2 * sms) * (zl + 2) * (yl + 1);
+        if (best == 0 || cost < best) {
+          best = cost;
+          nchunks = units;
+          P.yl = yl;
+          P.zl = zl;
+        }
+      }
+    }
     FCB_CUDA_TRY(cudaFuncSetAttribute(conv3d16n_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CVN_SMEM));
     const int grid = (int)std::min<long long>(nchunks, 2ll * sms);
     conv3d16n_kernel<<<grid, CVN_THREADS, CVN_SMEM, st>>>(map, P, (int)nchunks);
