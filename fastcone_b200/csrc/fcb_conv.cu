@@ -1226,12 +1226,10 @@ try {
     // the rows per walk and about one row's worth to start each pass; three rows at least (fewer
     // would wait for the epilogue).  64^3: 3 x 5, 22.3 us (5 x 3: 24.6); 256^3: 5 x 32.
     long long nchunks = 0, best = 0;
-    for (int yl = std::min(3, ny); yl <= std::min(CVN_Y, ny); yl++) {
-      const long long cols = (long long)P.tiles_x * ((ny + yl - 1) / yl);
-      const int least = (nz + 63) / 64, most = std::min(nz, least + 2 * sms);
-      for (int walks = least; walks <= most; walks++) {
-        const int zl = (nz + walks - 1) / walks;
-        const long long units = cols * ((nz + zl - 1) / zl);
+    for (int yl = std::min(3, ny); yl <= std::min(CVN_Y, ny); yl++)
+      for (int z = std::min(64, nz); z >= 1; z--) {
+        const int walks = (nz + z - 1) / z, zl = (nz + walks - 1) / walks;
+        const long long units = (long long)P.tiles_x * ((ny + yl - 1) / yl) * walks;
         const long long cost = (units + 2 * sms - 1) / (2 * sms) * (zl + 2) * (yl + 1);
         if (best == 0 || cost < best) {
           best = cost;
@@ -1240,7 +1238,6 @@ try {
           P.zl = zl;
         }
       }
-    }
     FCB_CUDA_TRY(cudaFuncSetAttribute(conv3d16n_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CVN_SMEM));
     const int grid = (int)std::min<long long>(nchunks, 2ll * sms);
     conv3d16n_kernel<<<grid, CVN_THREADS, CVN_SMEM, st>>>(map, P, (int)nchunks);
