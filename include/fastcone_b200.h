@@ -171,7 +171,8 @@ int fcb_project_device_counted(const fcb_geometry* g, int method, const float* v
                                float* proj, unsigned long long* samples, void* stream);
 
 /* Reusable backprojection plan (geometry digested once: per-view parameters, staging
- * window sizes).  execute() is asynchronous and allocates nothing. */
+ * window sizes).  execute() is asynchronous and allocates nothing but stream-ordered scratch for
+ * projection rows that are not whole 16-byte groups (without it they run unstaged). */
 typedef struct fcb_bp_plan fcb_bp_plan;
 int fcb_bp_plan_create(const fcb_geometry* g, int kernelMode, int projType, fcb_bp_plan** plan);
 int fcb_bp_plan_execute(fcb_bp_plan* plan, const void* proj, float* volume, void* stream);
@@ -234,7 +235,7 @@ int fcb_sync_status(void* stream);
 /* The host-buffer entry points (GPU_CB_*, fcb_backproject_host, fcb_project_host,
  * fcb_fbp_host) keep the device blocks of a finished call and reuse them in later calls
  * that fit (at most 8 blocks per device; a failed allocation first returns them), and
- * fcb_fbp_host keeps its filter plans (cuFFT plans and scratch, at most 4 per device).  This
+ * fcb_fbp_host keeps its filter plans (at most 4 per device).  This
  * returns everything kept to the driver.  FCB_HOST_CACHE=0 in the environment frees each
  * call's blocks and plans when it ends instead. */
 int fcb_release_device_cache(void);
