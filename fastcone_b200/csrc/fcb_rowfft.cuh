@@ -24,10 +24,12 @@
 // HBM.  A row's buffer limits how many rows an SM holds (13 of 1536 values), so latency is
 // hidden inside the warp: the next rows' values are loaded into registers while the current ones
 // are transformed, and the tables sit in shared memory (one persistent CTA per SM loads them
-// once).  1440 x 1024 rows of 1536 values, cosine weight and Shepp-Logan, on one B200: 13.8 ms
+// once).  1440 x 1024 rows of 1536 values, cosine weight and Shepp-Logan, on one B200: 14.2 ms
 // (21.4 ms with short-lived CTAs, tables through L1 and no prefetch); cuFFT R2C, a spectrum pass
-// and C2R between padding and cropping passes took 89.6 ms.  Error against 64 bits 4.3e-6 of the
-// result's norm there (cuFFT's 6.7e-6: the result is small against the smooth input).
+// and C2R between padding and cropping passes took 89.6 ms.  Error against 64 bits 4.2e-6 of the
+// result's norm there (cuFFT's 6.7e-6: the result is small against the smooth input); over 70
+// widths from 32 to 2048, smooth rows, Ram-Lak with and without the weight and Shepp-Logan, 0.38
+// to 0.91 of cuFFT's.
 //
 // The stages are functions of (thread, row buffer) so that the host can run them too.
 #pragma once
