@@ -6,11 +6,15 @@
 // crop to [0, W).  The apodised variants cosrampfilter / gaussrampfilter (fastcone.py:
 // 294-319) transform rows of length W unpadded.
 //
-// All of these are convolutions of a row with a fixed even kernel of W lags, so rows up to
+// The padded ones are convolutions of a row with a fixed even kernel of W lags, so rows up to
 // rf::RC_MAX_W values run in one kernel that reads and writes each projection once
 // (fcb_rowfft.cuh; the bound there is instruction issue and shared memory, not HBM).  Longer
 // rows keep cuFFT's batched R2C / C2R transforms with this file's pad / multiply / crop passes:
 // 64 x 256 rows of 4500 take 2.0 ms there, of 4096 0.41 ms in the one kernel (1.4 ms before).
+// So do the apodised variants at every width.  Their kernels, cyclic over W, do not decay, and as
+// linear convolutions over 2 W - 1 lags they carry twice the energy and its noise: on smooth rows the
+// one kernel was up to 2.2 times as far from 64 bits as cuFFT's transform of the row itself (113
+// values 2.2e-6 against 1.0e-6 of the norm, 1411 5.2e-6 against 3.7e-6).
 #include <cufft.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -118,7 +122,7 @@ struct FdkRows {
   }
 };
 
-// Rows longer than rf::RC_MAX_W: the three element-wise passes run on 2-D grids: x over a row's elements, y over the
+// The cuFFT form: the three element-wise passes run on 2-D grids: x over a row's elements, y over the
 // batch's rows (at most 65535), so no thread divides its index.  (Measured against the
 // earlier one-dimensional form, which divided a 64-bit index per element: the same 2-4 TB/s;
 // these passes are a third of the filter's time, cuFFT the rest.)
@@ -220,12 +224,13 @@ __global__ void phantom_kernel(const __grid_constant__ PhParams P, int e0)
 
 using namespace fcb;
 
-// Reusable filter: the row transform's tables (long rows: cuFFT plans, padded rows, spectra and
-// the filter response) made once; execute() is stream-ordered, allocates nothing and does not
+// Reusable filter: the row transform's tables (long rows and the unpadded windows: cuFFT plans, rows,
+// spectra and the filter response) made once; execute() is stream-ordered, allocates nothing and does not
 // synchronise.
 struct fcb_filter_plan {
   int nviews = 0, H = 0, W = 0, outType = FCB_F32, window = FCB_FILTER_RAMLAK;
-  rf::RowConv conv;  // rows up to rf::RC_MAX_W; the members below serve longer ones
+  bool fused = false;  // padded rows up to rf::RC_MAX_W: `conv`; the members below serve the others
+  rf::RowConv conv;
   int n2 = 0, nb = 0, batch = 0;
   float* pad = nullptr;
   cufftComplex* spec = nullptr;
@@ -305,7 +310,8 @@ try {
   pl->nviews = nviews; pl->H = H; pl->W = W; pl->outType = outType; pl->window = window;
   pl->n2 = L;
   pl->nb = L / 2 + 1;
-  if (W <= rf::RC_MAX_W) {
+  pl->fused = L == 2 * W && W <= rf::RC_MAX_W;
+  if (pl->fused) {
     int rc = pl->conv.create(W, filt.data(), pl->nb, L);
     if (rc == FCB_OK && cudaMalloc(&pl->dz, nviews * sizeof(float)) != cudaSuccess) {
       cudaGetLastError();
@@ -374,7 +380,7 @@ int filter_plan_run(fcb_filter_plan* pl, const float* in, void* out, int nviews,
   if (cosineWeight && (!dzorig || !(D > 0.0f)))
     return set_error(FCB_ERR_INVALID, "cosine weighting needs D > 0 and zOrigin");
   const int n2 = pl->n2, nb = pl->nb, W = pl->W, H = pl->H, batch = pl->batch;
-  if (W <= rf::RC_MAX_W) {
+  if (pl->fused) {
     const int es = dtype_size(pl->outType);
     FdkRows io{in, out, dzorig, D, pl->outType, H, W, pitch, cosineWeight ? 1 : 0, 0, 0};
     io.vin = pitch % 2 == 0 && (uintptr_t)in % 8 == 0;
