@@ -49,7 +49,7 @@ int device_status_ptr(int** p)
 // The one-shot entry points need device scratch for the length of a call (a copy of the volume,
 // a window table).  CUDA's default pool gives freed memory back to the driver at the next
 // synchronisation, so calls that synchronise once mapped their scratch anew each time: 0.5 to
-// 1 ms of a 64^3 projection.  A pool of the library's own, one per device, keeps up to
+// 1 ms of a 64^3 projection.  A pool of the library's own, one per device and context, keeps up to
 // POOL_KEEP bytes instead.  The allocator orders reuse by stream, so calls on several streams
 // and threads are safe; scratch_trim returns what is idle.
 namespace {
@@ -62,7 +62,9 @@ struct ScratchPool {
 std::mutex g_pool_mu;
 std::vector<ScratchPool> g_pools;
 
-// The current device's pool; null where pools are not supported.
+// The current context's pool; null where pools are not supported.  Entries stay: several contexts of
+// a device may live side by side, and the entry of one that was reset is never asked for again (its
+// id is not given out twice).
 cudaMemPool_t scratch_pool()
 {
   int dev = 0, supported = 0;
@@ -72,12 +74,8 @@ cudaMemPool_t scratch_pool()
   }
   const unsigned long long ctx = current_context_id();
   std::lock_guard<std::mutex> lk(g_pool_mu);
-  for (size_t i = 0; i < g_pools.size();) {
-    if (g_pools[i].dev == dev && g_pools[i].ctx == ctx) return g_pools[i].pool;
-    // a pool of a context that is gone went with it
-    if (g_pools[i].dev == dev) g_pools.erase(g_pools.begin() + (long)i);
-    else i++;
-  }
+  for (const ScratchPool& q : g_pools)
+    if (q.dev == dev && q.ctx == ctx) return q.pool;
   cudaMemPool_t pool = nullptr;
   if (cudaDeviceGetAttribute(&supported, cudaDevAttrMemoryPoolsSupported, dev) == cudaSuccess && supported) {
     cudaMemPoolProps props;
@@ -122,10 +120,20 @@ void scratch_trim()
 {
   int cur = -1;
   cudaGetDevice(&cur);
+  const unsigned long long ctx = current_context_id();
+  bool moved = false;
   std::lock_guard<std::mutex> lk(g_pool_mu);
-  for (const ScratchPool& q : g_pools)
+  for (const ScratchPool& q : g_pools) {
+    // on the caller's device its own context's pool (cudaSetDevice would leave a context that is not the
+    // primary one), on the others their primary context's
+    if (q.dev == cur) {
+      if (q.ctx == ctx) cudaMemPoolTrimTo(q.pool, 0);
+      continue;
+    }
+    moved = true;
     if (cudaSetDevice(q.dev) == cudaSuccess && current_context_id() == q.ctx) cudaMemPoolTrimTo(q.pool, 0);
-  if (cur >= 0) cudaSetDevice(cur);
+  }
+  if (moved && cur >= 0) cudaSetDevice(cur);
   cudaGetLastError();
 }
 
