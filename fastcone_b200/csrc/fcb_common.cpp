@@ -95,7 +95,11 @@ cudaMemPool_t scratch_pool()
 
 int scratch_alloc(void** p, size_t bytes, cudaStream_t st)
 {
-  cudaMemPool_t pool = scratch_pool();
+  // Under capture the allocation becomes a node of the graph with memory of the graph's own, and
+  // making a context or a pool (even cudaFree(nullptr)) would invalidate the capture.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+  cudaMemPool_t pool = cap == cudaStreamCaptureStatusNone ? scratch_pool() : nullptr;
   cudaError_t e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, st) : cudaMallocAsync(p, bytes, st);
   if (e != cudaSuccess && pool) {
     cudaGetLastError();
