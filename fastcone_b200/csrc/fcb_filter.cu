@@ -295,6 +295,12 @@ static int filter_response(int W, int window, double gaussScale, int* L, std::ve
   return FCB_OK;
 }
 
+// Rows per cuFFT batch: about 256 MB of padded rows, at most 65535 (the kernels' grid y).
+static long long filter_batch_rows(long long rows, int n2)
+{
+  return std::min<long long>(std::min<long long>(rows, 65535), std::max<long long>(1, (256ll << 20) / (8ll * n2)));
+}
+
 extern "C" int fcb_filter_plan_create_ex(int nviews, int H, int W, int outType, int window,
                                          double gaussScale, fcb_filter_plan** out)
 try {
@@ -326,9 +332,7 @@ try {
   }
   const std::vector<float> filt32(filt.begin(), filt.end());
   const long long rows = (long long)nviews * H;
-  // rows per cuFFT batch: about 256 MB of padded rows, at most 65535 (the kernels' grid y)
-  pl->batch = (int)std::min<long long>(std::min<long long>(rows, 65535),
-                                       std::max<long long>(1, (256ll << 20) / (8ll * pl->n2)));
+  pl->batch = (int)filter_batch_rows(rows, pl->n2);
   int rc = FCB_OK;
   do {
     if (cudaMalloc(&pl->pad, (size_t)pl->batch * pl->n2 * sizeof(float)) != cudaSuccess ||
@@ -368,9 +372,11 @@ FCB_CATCH_STATUS
 
 namespace fcb {
 // Filters the first `nviews` (<= the plan's) views of `in` into `out`, both with rows of the
-// plan's W values at a pitch of `pitch` elements (in == out allowed for FP32 output).
+// plan's W values at a pitch of `pitch` elements.
 // dzorig: device array of the views' zOrigin (cosine weight), or NULL without weighting.
-// Stream-ordered, no allocation.
+// Stream-ordered, no allocation unless the buffers overlap in another way than FP32 in place: the
+// row transform writes rows while others are still to be read, so such rows go through a copy, as
+// many at a time as the cuFFT form takes (which reads a batch before it writes it).
 int filter_plan_run(fcb_filter_plan* pl, const float* in, void* out, int nviews, int pitch, float D,
                     const float* dzorig, int cosineWeight, cudaStream_t st)
 {
@@ -385,7 +391,28 @@ int filter_plan_run(fcb_filter_plan* pl, const float* in, void* out, int nviews,
     FdkRows io{in, out, dzorig, D, pl->outType, H, W, pitch, cosineWeight ? 1 : 0, 0, 0};
     io.vin = pitch % 2 == 0 && (uintptr_t)in % 8 == 0;
     io.vout = pitch % 2 == 0 && (uintptr_t)out % (2 * es) == 0;
-    return pl->conv.run<false>(io, (long long)nviews * H, st);
+    const long long rows = (long long)nviews * H;
+    const long long values = (rows - 1) * pitch + W;
+    const uintptr_t in0 = (uintptr_t)in, in1 = in0 + values * sizeof(float);
+    const uintptr_t out0 = (uintptr_t)out, out1 = out0 + values * es;
+    if (in1 <= out0 || out1 <= in0 || (in0 == out0 && pl->outType == FCB_F32))
+      return pl->conv.run<false>(io, rows, st);
+    const long long nr = filter_batch_rows(rows, n2);
+    float* copy = nullptr;
+    FCB_TRY(scratch_alloc((void**)&copy, (size_t)nr * pitch * sizeof(float), st));
+    io.vin = pitch % 2 == 0;
+    int rc = FCB_OK;
+    for (long long r0 = 0; r0 < rows && rc == FCB_OK; r0 += nr) {
+      const long long n = std::min(nr, rows - r0);
+      const cudaError_t e = cudaMemcpyAsync(copy, in + r0 * pitch, ((n - 1) * pitch + W) * sizeof(float),
+                                            cudaMemcpyDeviceToDevice, st);
+      if (e != cudaSuccess) rc = set_error(FCB_ERR_CUDA, cudaGetErrorString(e));
+      // (where row 0 would be: only rows from r0 on are read)
+      io.in = reinterpret_cast<const float*>((uintptr_t)copy - (uintptr_t)(r0 * pitch) * sizeof(float));
+      if (rc == FCB_OK) rc = pl->conv.run<false>(io, n, st, r0);
+    }
+    scratch_free(copy, st);
+    return rc;
   }
   if (cufftSetStream(pl->pf, st) != CUFFT_SUCCESS || cufftSetStream(pl->pi, st) != CUFFT_SUCCESS)
     return set_error(FCB_ERR_CUDA, "cufftSetStream failed");

@@ -601,19 +601,19 @@ struct RowConv {
     rc_dispatch(W, [&](auto k) { n = (long long)decltype(k)::GPC * decltype(k)::R * sms; });
     return n;
   }
-  // Convolves `nrows` rows through `io`, stream-ordered.
+  // Convolves `nrows` rows from row `first` on through `io`, stream-ordered.
   template <bool ODD, class IO>
-  int run(const IO& io, long long nrows, cudaStream_t st) const
+  int run(const IO& io, long long nrows, cudaStream_t st, long long first = 0) const
   {
     int rc = FCB_OK;
     rc_dispatch(W, [&](auto k) {
       using K = decltype(k);
-      rc = launch<K, ODD>(io, nrows, st);
+      rc = launch<K, ODD>(io, nrows, st, first);
     });
     return rc;
   }
   template <class K, bool ODD, class IO>
-  int launch(const IO& io, long long nrows, cudaStream_t st) const
+  int launch(const IO& io, long long nrows, cudaStream_t st, long long first) const
   {
     auto kern = rowconv_kernel<K, ODD, IO>;
     FCB_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, K::SMEM));
@@ -624,7 +624,7 @@ struct RowConv {
       const int n = (int)(nrows - r0 < (1 << 30) ? nrows - r0 : (1 << 30));
       const int units = (n + K::R - 1) / K::R;
       kern<<<(unsigned)(units < sms ? units : sms), K::T * K::GPC, K::SMEM, st>>>(
-          io, reinterpret_cast<const uint4*>(block), r0, n);
+          io, reinterpret_cast<const uint4*>(block), first + r0, n);
       FCB_CUDA_TRY(cudaGetLastError());
     }
     return FCB_OK;

@@ -186,7 +186,8 @@ class FilterPlan:
     """Reusable FDK filter (cosine weight + ramp / Shepp-Logan, or the unpadded cosine /
     Gaussian apodised ramps with ``window=FILTER_COSRAMP / FILTER_GAUSSRAMP``) for projections of shape
     (nviews, H, W): tables (apodised windows and rows above 4096 values: cuFFT plans and scratch)
-    made once; calls are stream-ordered, allocate nothing and do not synchronise."""
+    made once; calls are stream-ordered, do not synchronise and allocate nothing (unless ``out``
+    overlaps the input in another way than FP32 in place)."""
 
     def __init__(self, shape, out_dtype=torch.float32, window: int = _lib.FILTER_RAMLAK,
                  gauss_scale: float = 0.125):

@@ -253,8 +253,9 @@ int fcb_fdk_filter_device(const float* in, void* out, int outType, int nviews, i
 
 /* The same filter as a reusable plan: the row transform's tables (apodised windows and rows above
  * 4096 values: cuFFT plans, scratch and the filter response) are made once; execute is
- * stream-ordered, allocates nothing and does not synchronise (zOrigin, host, is read before it
- * returns).  One execute at a time per plan (the scratch is the plan's). */
+ * stream-ordered, allocates nothing (unless in and out overlap in another way than FP32 in place:
+ * then a stream-ordered copy of up to 64 MiB of in) and does not synchronise (zOrigin, host, is
+ * read before it returns).  One execute at a time per plan (the scratch is the plan's). */
 typedef struct fcb_filter_plan fcb_filter_plan;
 int fcb_filter_plan_create(int nviews, int H, int W, int outType, int window,
                            fcb_filter_plan** plan);
