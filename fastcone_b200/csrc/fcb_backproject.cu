@@ -79,11 +79,18 @@ struct FdkParams {
   unsigned long long cwait_ns;
   int stop_after;
   int pbufs;                    // 16-bit storage: tap-pair buffers (fdk_pair_kernel)
-  const GenView* gen;           // MATRIX kernels: the launch's views as the generic kernel has them
-  FdkView v[FDK_MAXV];
+  __align__(16) FdkView v[FDK_MAXV];  // MATRIX kernels: nviews of them, then the same views as GenView
 };
 
 static_assert(sizeof(FdkParams) + sizeof(CUtensorMap) < 32000, "kernel parameter space");
+
+// Views of a MATRIX launch.  Its parameters carry both forms of a view, so that the matrices are in
+// place when the kernel is, whatever stream it runs on, and a plan needs no device memory for them.
+constexpr int MATRIX_MAXV = FDK_MAXV * sizeof(FdkView) / (sizeof(FdkView) + sizeof(GenView));
+__host__ __device__ __forceinline__ const GenView* matrix_views(const FdkParams& P)
+{
+  return reinterpret_cast<const GenView*>(P.v + P.nviews);
+}
 
 __device__ __forceinline__ void fdk_footprint(const FdkParams& P, const FdkView& V, float x0,
                                               float x1, float y0, float y1, float z0, float z1,
@@ -631,9 +638,9 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
         }
         if (nw > P.BW || nh > P.BH) dev::record_status(P.status, DEV_RANGE);
         origin[s] = make_int4(__float_as_int((float)w0), __float_as_int((float)h0), v, nh);
-        if constexpr (!MATRIX) vstage[s] = P.v[v];
-        dev::mbar_arrive_expect_tx(&full[s], bytes + (MATRIX ? (uint32_t)sizeof(GenView) : 0u));
-        if constexpr (MATRIX) dev::bulk_load(&gstage[s], P.gen + v, (uint32_t)sizeof(GenView), &full[s]);
+        if constexpr (MATRIX) gstage[s] = matrix_views(P)[v];
+        else vstage[s] = P.v[v];
+        dev::mbar_arrive_expect_tx(&full[s], bytes);
         dev::tma_load_3d(smem_raw + (size_t)s * stage_bytes, &tmap, &full[s], w0, h0, P.view0 + v);
         issued++;
         if (++ps == P.stages) { ps = 0; pround ^= 1u; }
@@ -1024,7 +1031,7 @@ __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_c
       }
       if constexpr (MATRIX)
         if (lane < (int)(sizeof(GenView) / sizeof(float4)))
-          reinterpret_cast<float4*>(gpair + p)[lane] = __ldg(reinterpret_cast<const float4*>(P.gen + o.z) + lane);
+          reinterpret_cast<float4*>(gpair + p)[lane] = reinterpret_cast<const float4*>(matrix_views(P) + o.z)[lane];
       __syncwarp();
       dev::mbar_arrive(&full2[p]);  // all 32 lanes: their writes are released to the consumers
       conv++;
@@ -1440,11 +1447,10 @@ struct fcb_bp_plan {
   std::vector<GenParams> gen;
   std::vector<int> gen_parent;  // the view chunk (launch of `fdk`, or itself) each `gen` entry belongs to
   int4* d_win = nullptr;  // reference-compatible window table (device), when in use
-  GenView* d_gen = nullptr;  // rows that TMA cannot describe: the views' matrices (device)
+  std::vector<GenView> matrices;  // rows that TMA cannot describe: all views as launch_matrix wants them
   ~fcb_bp_plan()
   {
     if (d_win) cudaFree(d_win);
-    if (d_gen) cudaFree(d_gen);
   }
 };
 
@@ -1590,7 +1596,7 @@ int execute_repacked(fcb_bp_plan* pl, int chunk, int tz0, int tz1, const void* p
   const int W = pl->pb.projWHSize[0], H = pl->pb.projWHSize[1], es = (int)sizeof(T);
   const int pitch = (W * es + 15) / 16 * 16 / es;
   int maxv = 0;
-  for (const FdkParams& F : pl->fdk) maxv = std::max(maxv, F.nviews);
+  for (const FdkParams& F : pl->fdk) maxv = std::max(maxv, std::min(F.nviews, MATRIX_MAXV));
   void* buf = nullptr;
   if (scratch_alloc(&buf, (size_t)maxv * H * pitch * es, st) != FCB_OK) return ok();
   int rc = FCB_OK;
@@ -1598,19 +1604,24 @@ int execute_repacked(fcb_bp_plan* pl, int chunk, int tz0, int tz1, const void* p
     const FdkParams& F = pl->fdk[c];
     const int layer = F.tiles_x * F.tiles_y, ntiles = (tz1 - tz0) * layer;
     if ((chunk >= 0 && c != chunk) || ntiles <= 0) continue;
-    const long long rows = (long long)F.nviews * H;
-    repack_rows_kernel<T><<<dim3((unsigned)((W + 127) / 128), (unsigned)std::min<long long>(rows, 16384)), 128, 0, st>>>(
-        reinterpret_cast<const T*>(proj) + (size_t)F.view0 * H * W, reinterpret_cast<T*>(buf), W, pitch, rows);
-    CUtensorMap map;
-    rc = encode_tmap_3d(&map, tmap_type(pl->ptype), buf, W, H, F.nviews, (uint64_t)pitch * es,
-                        (uint64_t)pitch * H * es, pl->BW, pl->BH, 1);
-    if (rc) break;
-    FdkParams P = F;
-    P.vol = volume;
-    P.tile0 = tz0 * layer;
-    P.gen = pl->d_gen + F.view0;
-    P.view0 = 0;
-    rc = launch_matrix<T>(pl, map, P, ntiles, st);
+    for (int k = 0; k < F.nviews && rc == FCB_OK; k += MATRIX_MAXV) {
+      const int n = std::min(MATRIX_MAXV, F.nviews - k), v0 = F.view0 + k;
+      const long long rows = (long long)n * H;
+      repack_rows_kernel<T><<<dim3((unsigned)((W + 127) / 128), (unsigned)std::min<long long>(rows, 16384)), 128, 0, st>>>(
+          reinterpret_cast<const T*>(proj) + (size_t)v0 * H * W, reinterpret_cast<T*>(buf), W, pitch, rows);
+      CUtensorMap map;
+      rc = encode_tmap_3d(&map, tmap_type(pl->ptype), buf, W, H, n, (uint64_t)pitch * es, (uint64_t)pitch * H * es,
+                          pl->BW, pl->BH, 1);
+      if (rc) break;
+      FdkParams P = F;
+      P.vol = volume;
+      P.tile0 = tz0 * layer;
+      P.view0 = 0;
+      P.nviews = n;
+      memmove(P.v, P.v + k, n * sizeof(FdkView));
+      memcpy(P.v + n, pl->matrices.data() + v0, n * sizeof(GenView));
+      rc = launch_matrix<T>(pl, map, P, ntiles, st);
+    }
   }
   scratch_free(buf, st);
   *done = true;
@@ -1868,15 +1879,8 @@ static int bp_plan_build(const fcb_geometry* g, int kernelMode, int projType, in
   if (pl->path == 1 && may_alloc && !piwin && pl->nz_tile == 32 &&
       ((size_t)pb.projWHSize[0] * dtype_size(projType)) % 16 != 0) {
     // rows that TMA cannot describe: the matrices that the staged kernels then take positions from
-    std::vector<GenView> gv((size_t)pb.nviews);
-    fill_gen_views(pb, 0, pb.nviews, gv.data());
-    if (cudaMalloc(&pl->d_gen, gv.size() * sizeof(GenView)) != cudaSuccess) {
-      cudaGetLastError();
-      pl->d_gen = nullptr;  // the generic kernel needs none
-    } else if (cudaMemcpy(pl->d_gen, gv.data(), gv.size() * sizeof(GenView), cudaMemcpyHostToDevice) != cudaSuccess) {
-      delete pl;
-      return set_error(FCB_ERR_CUDA, "copy of the view matrices failed");
-    }
+    pl->matrices.resize((size_t)pb.nviews);
+    fill_gen_views(pb, 0, pb.nviews, pl->matrices.data());
   }
   if (pl->path == 0) {
     const int gmax = std::min(GEN_MAXV, pl->maxv);
@@ -1992,7 +1996,7 @@ int bp_plan_execute_range(fcb_bp_plan* pl, int chunk, int z0, int z1, const void
     }
     return ok();
   }
-  if (pl->path == 1 && pl->d_gen && (uintptr_t)proj % es == 0) {
+  if (pl->path == 1 && !pl->matrices.empty() && (uintptr_t)proj % es == 0) {
     // (not under capture: the scratch would become part of the graph)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     FCB_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
