@@ -1416,8 +1416,11 @@ __global__ void pi_pairs_kernel(const PiView* __restrict__ views, int nviews, in
 // A tensor map wants a 16-byte aligned base and row strides of whole 16 bytes.  Projections of
 // other widths are copied, a launch's views at a time, to rows at a pitch that has them (the map
 // keeps the true width, so the padding is never read).  251 x 237 x 203 voxels, 200 views of
-// 379 x 231, on one B200: 2.02 ms with the copies and the matrix positions, 11.5 ms by the generic
-// kernel's global gathers (the same bits), 1.77 ms for rows of 380.
+// 379 x 231, on one B200: 2.00 ms with the copies and the matrix positions, 11.5 ms by the generic
+// kernel's global gathers, 1.77 ms for rows of 380.  Positions and weights are the generic kernel's bit
+// for bit, and with one CTA per tile so are the sums; where the CTAs of a cluster share a tile's views
+// (split_ranks) the views are added in their parts, and a captured call, which runs the generic kernel,
+// differs by the rounding of the sums.
 namespace fcb {
 template <typename T>
 __global__ void repack_rows_kernel(const T* __restrict__ in, T* __restrict__ out, int W, int pitch, long long rows)

@@ -172,7 +172,11 @@ int fcb_project_device_counted(const fcb_geometry* g, int method, const float* v
 
 /* Reusable backprojection plan (geometry digested once: per-view parameters, staging
  * window sizes).  execute() is asynchronous and allocates nothing but stream-ordered scratch for
- * projection rows that are not whole 16-byte groups (without it they run unstaged). */
+ * projection rows that are not whole 16-byte groups (without it, and under capture, such rows run
+ * unstaged).  The order in which a voxel's views are added depends on the number of tiles of the
+ * launch (small volumes: partial sums of up to 8 parts of the views) and on that route, so results of
+ * other sub-volumes, of a captured and of a direct call may differ by the rounding of the sums; the
+ * same call repeats bit for bit. */
 typedef struct fcb_bp_plan fcb_bp_plan;
 int fcb_bp_plan_create(const fcb_geometry* g, int kernelMode, int projType, fcb_bp_plan** plan);
 int fcb_bp_plan_execute(fcb_bp_plan* plan, const void* proj, float* volume, void* stream);

@@ -78,3 +78,27 @@ def test_launches_of_many_views(views, monkeypatch):
     ops.sync_status()
     # the same terms in other partial sums: a rounding per term at most, random signs
     assert float((got - ref).abs().max()) < 64 * 2.0 ** -24 * 4.0 * np.sqrt(views)
+
+
+@pytest.mark.parametrize("dtype", ["float32", "float16", "bfloat16"])
+@pytest.mark.parametrize("vol,views", [((33, 30, 27), 250), ((64, 64, 64), 181)])
+def test_captured_calls_agree_to_rounding(vol, views, dtype):
+    """A captured call runs the generic kernel, which adds the views in one order; an eager call of few
+    tiles adds them in the parts of a cluster's CTAs: equal but for the rounding of the sums."""
+    import torch
+
+    from fastcone_b200 import ops
+
+    g, _ = make_case(vol_xyz=vol, det_wh=(97, 50), nviews=views, D=260.0, pw=0.8)
+    dt = getattr(torch, dtype)
+    proj = torch.randn(g.proj_shape, device="cuda").to(dt)
+    plan = ops.BackprojectPlan(g, mode=2, dtype=dt)
+    eager = plan(proj, torch.zeros(g.vol_shape, device="cuda"))
+    out = torch.zeros(g.vol_shape, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan(proj, out)
+    out.zero_()
+    graph.replay()
+    ops.sync_status()
+    assert float((eager - out).abs().max()) < 64 * 2.0 ** -24 * 4.0 * np.sqrt(views)
