@@ -461,7 +461,7 @@ constexpr int CVN_STAGE = (CVN_Y + 2) * 2 * (CV_ROW + 2) * 16;  // [row][channel
 constexpr int CVN_WB = 80 * 32;            // weights of one (dy, dx): [K half][dz = 2, 1, 0, 2, 1][16 out] x 16 B
 constexpr int CVN_COLS = 256;              // TMEM columns (48 a row): two CTAs per SM
 constexpr int CVN_ACC = 3 * CVN_Y;         // accumulator blocks
-constexpr int CVN_SMEM = CVN_STAGES * CVN_STAGE + 9 * CVN_WB + 64 + 8 * (2 * CVN_STAGES + 2 * CVN_ACC) + 16;
+constexpr int CVN_SMEM = CVN_STAGES * CVN_STAGE + 9 * CVN_WB + 64 + 8 * (2 * CVN_STAGES + 2 * CVN_ACC + 1) + 16;
 static_assert(CVN_STAGE % 128 == 0 && 3 * CVN_SMEM > 227 * 1024 && 2 * (CVN_SMEM + 1024) <= 228 * 1024 &&
                   16 * CVN_ACC <= CVN_COLS && 2 * CVN_COLS <= 512,
               "two CTAs per SM");
@@ -492,7 +492,8 @@ __global__ void __launch_bounds__(CVN_THREADS, 2) conv3d16n_kernel(const __grid_
   uint64_t* empty = full + CVN_STAGES;
   uint64_t* accf = empty + CVN_STAGES;  // [CVN_ACC] row of a plane complete (MMA commit)
   uint64_t* acce = accf + CVN_ACC;      // [CVN_ACC] row read and cleared (4 epilogue warps)
-  uint32_t* tslot = reinterpret_cast<uint32_t*>(acce + CVN_ACC);
+  uint64_t* fin = acce + CVN_ACC;       // every MMA issued is complete, after a wait that ran out
+  uint32_t* tslot = reinterpret_cast<uint32_t*>(fin + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const ConvChunks CH{P.tiles_x, P.ny, P.nz, P.yl, P.zl, (P.ny + P.yl - 1) / P.yl};
@@ -506,6 +507,7 @@ __global__ void __launch_bounds__(CVN_THREADS, 2) conv3d16n_kernel(const __grid_
       dev::mbar_init(&accf[q], 1);
       dev::mbar_init(&acce[q], 4);
     }
+    dev::mbar_init(fin, 1);
     dev::fence_mbar_init();
   }
   if (warp == 5) {
@@ -621,8 +623,14 @@ __global__ void __launch_bounds__(CVN_THREADS, 2) conv3d16n_kernel(const __grid_
           if (++s == CVN_STAGES) { s = 0; ph ^= 1u; }
         }
       }
-      // every MMA issued must be complete before the columns are released: the last stage's commit
-      if (stages > 0) dev::mbar_wait(&empty[(stages - 1) % CVN_STAGES], ((stages - 1) / CVN_STAGES) & 1, 100000000ull);
+      // every MMA issued must be complete before the columns are released: the last stage's commit, or,
+      // where a plane was given up halfway, one behind them all
+      if (failed) {
+        tc::mma_commit(fin);
+        dev::mbar_wait(fin, 0, 100000000ull);
+      } else if (stages > 0) {
+        dev::mbar_wait(&empty[(stages - 1) % CVN_STAGES], ((stages - 1) / CVN_STAGES) & 1, 100000000ull);
+      }
     }
   } else {
     // ---------------------------------------------------------------- epilogue (warps 0-3)
