@@ -104,12 +104,13 @@ __device__ __forceinline__ KatsColumn kats_column(const float* m, const float* c
   X.q2d = X.q2 * K.iD;
   return X;
 }
-// The derivative at fixed ray direction and the length correction at row j.  (32-bit indices
-// from the views' uniform base addresses.)
+// The derivative at fixed ray direction and the length correction at row j.  I indexes a view from
+// its uniform base address: 32 bits where they hold its H W values.
+template <typename I>
 __device__ __forceinline__ float kats_deriv(const KatsColumn& X, int j, int H, int W, const KatsDerivConst& K)
 {
-  const unsigned o = (unsigned)(j * W + X.i);
-  const unsigned up = j > 0 ? o - W : o, dn = j < H - 1 ? o + W : o;
+  const I o = (I)j * (I)W + (I)X.i;
+  const I up = j > 0 ? o - (I)W : o, dn = j < H - 1 ? o + (I)W : o;
   const float dl = (X.p[o] - X.m[o]) * X.sl;
   const float dgu = (X.c[o + X.dr] - X.c[o + X.dl]) * X.su;
   const float dgv = (X.c[dn] - X.c[up]) * (j > 0 && j < H - 1 ? K.hipw : K.ipw);
@@ -124,9 +125,9 @@ __device__ __forceinline__ float kats_deriv(const KatsColumn& X, int j, int H, i
 // The strip's derivatives of one view sit in shared memory between the two (STAGE), since each is
 // read about 2 K / H times (the strip takes 128 bytes a row: up to 768 rows leave two CTAs per SM);
 // beyond that every tap is derived where it is read.
-// `before` is view t0 - 1 (null at the first view).
+// `before` is view t0 - 1 (null at the first view).  I: as in kats_deriv, for the K L values too.
 constexpr int KK_VIEWS = 4;
-template <bool STAGE>
+template <bool STAGE, typename I>
 __global__ void __launch_bounds__(256, 5) kats_kappa_kernel(const float* __restrict__ g,
                                                             const float* __restrict__ before,
                                                             float* __restrict__ out, const float2* __restrict__ tab,
@@ -146,7 +147,7 @@ __global__ void __launch_bounds__(256, 5) kats_kappa_kernel(const float* __restr
     if constexpr (STAGE) {
       if (i < W) {
 #pragma unroll 2
-        for (int j = warp; j < H; j += 8) kk_g2[j * 32 + lane] = kats_deriv(X, j, H, W, C);
+        for (int j = warp; j < H; j += 8) kk_g2[j * 32 + lane] = kats_deriv<I>(X, j, H, W, C);
       }
       __syncthreads();
     }
@@ -154,15 +155,15 @@ __global__ void __launch_bounds__(256, 5) kats_kappa_kernel(const float* __restr
       float* row = out + (size_t)tl * K * L;
 #pragma unroll 4
       for (int k = warp; k < K; k += 8) {
-        const float2 ja = __ldg(tab + (unsigned)(k * W + i));
+        const float2 ja = __ldg(tab + ((I)k * (I)W + (I)i));
         const int j0 = __float_as_int(ja.x);
         float val = 0.0f;
         if (j0 >= 0) {  // (and at most H - 2)
-          const float v0 = STAGE ? kk_g2[j0 * 32 + lane] : kats_deriv(X, j0, H, W, C);
-          const float v1 = STAGE ? kk_g2[j0 * 32 + lane + 32] : kats_deriv(X, j0 + 1, H, W, C);
+          const float v0 = STAGE ? kk_g2[j0 * 32 + lane] : kats_deriv<I>(X, j0, H, W, C);
+          const float v1 = STAGE ? kk_g2[j0 * 32 + lane + 32] : kats_deriv<I>(X, j0 + 1, H, W, C);
           val = fmaf(ja.y, v1 - v0, v0);
         }
-        row[(unsigned)(k * L + i)] = val;
+        row[(I)k * (I)L + (I)i] = val;
       }
     }
     if constexpr (STAGE) __syncthreads();
@@ -483,16 +484,17 @@ try {
   }
   const size_t strip = (size_t)H * 32 * sizeof(float);  // a view's derivatives in 32 columns
   const bool stage = strip <= 96 * 1024;
-  if (stage)
-    FCB_CUDA_TRY(cudaFuncSetAttribute(kats_kappa_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+  const bool wide = std::max((long long)H * W, (long long)K * L) > 0x7fffffffll;
+  auto kappa = stage ? (wide ? kats_kappa_kernel<true, size_t> : kats_kappa_kernel<true, unsigned>)
+                     : (wide ? kats_kappa_kernel<false, size_t> : kats_kappa_kernel<false, unsigned>);
+  if (stage) FCB_CUDA_TRY(cudaFuncSetAttribute(kappa, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
   // one batch: kappa rows of views [t0, t0 + nv), their Hilbert transform, backward rebinning
   auto batch = [&](int t0, int nv) -> int {
     const long long rows = (long long)nv * K;
     float* g3 = fused || direct ? pl->g4 : pl->g3;
     const float* before = t0 == 0 ? nullptr : in == out ? pl->edge : src + (size_t)(t0 - 1) * plane;
     const dim3 kg((W + 31) / 32, (nv + KK_VIEWS - 1) / KK_VIEWS);
-    if (stage) kats_kappa_kernel<true><<<kg, 256, strip, st>>>(src, before, g3, pl->dfja, nviews, H, W, K, L, t0, nv, KC);
-    else kats_kappa_kernel<false><<<kg, 256, 0, st>>>(src, before, g3, pl->dfja, nviews, H, W, K, L, t0, nv, KC);
+    kappa<<<kg, 256, stage ? strip : 0, st>>>(src, before, g3, pl->dfja, nviews, H, W, K, L, t0, nv, KC);
     FCB_CUDA_TRY(cudaGetLastError());
     if (in == out && t0 + nv < nviews)
       FCB_CUDA_TRY(cudaMemcpyAsync(pl->edge, in + (size_t)(t0 + nv - 1) * plane, plane * sizeof(float),
