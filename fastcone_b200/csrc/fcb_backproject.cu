@@ -554,7 +554,7 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
   static_assert(!SPLIT || X2, "split views");
   const uint32_t rank = SPLIT ? cluster_rank() : 0, nrank = SPLIT ? cluster_size() : 1;
   fdk_tile(P, P.tile0 + (SPLIT ? blockIdx.x / nrank : blockIdx.x), tx, ty, tz);
-  int v0 = 0, v1 = P.nviews;  // this CTA's views (PI window: every nrank-th batch of 32)
+  int v0 = 0, v1 = P.nviews;  // this CTA's views (PI window: every nrank-th)
   if constexpr (SPLIT && !PIW) split_views(P.nviews, rank, nrank, &v0, &v1);
 
   if (threadIdx.x == 0) {
@@ -575,10 +575,11 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
     bool failed = false, stalled = false;
     if constexpr (PIW) {
       // the whole warp tests 32 views at a time against the PI window (most views miss a
-      // tile of a helical scan); lane 0 stages the ones that reach it, in view order
+      // tile of a helical scan); lane 0 stages the ones that reach it, in view order (SPLIT: every
+      // nrank-th view, since those that reach a tile follow each other)
       if (lane == 0) dev::tma_prefetch(&tmap);
-      for (int vb = 32 * (int)rank; vb < P.nviews && !failed && !stalled; vb += 32 * (int)nrank) {
-        const int v = vb + lane;
+      for (int vb = (int)rank; vb < P.nviews && !failed && !stalled; vb += 32 * (int)nrank) {
+        const int v = vb + lane * (int)nrank;
         int w0 = 0, h0 = 0, nw = 0, nh = 0;
         bool need = false;
         if (v < P.nviews) {
@@ -592,7 +593,7 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
             stalled = true;
             break;
           }
-          const int l = __ffs(mask) - 1;
+          const int l = __ffs(mask) - 1, vl = vb + l * (int)nrank;
           mask &= mask - 1;
           const int sw0 = __shfl_sync(0xffffffffu, w0, l), sh0 = __shfl_sync(0xffffffffu, h0, l);
           const int snw = __shfl_sync(0xffffffffu, nw, l), snh = __shfl_sync(0xffffffffu, nh, l);
@@ -603,11 +604,10 @@ __global__ void __launch_bounds__(FDK_THREADS, MINB) fdk_tma_kernel(const __grid
               ok = 0;
             } else {
               if (snw > P.BW || snh > P.BH) dev::record_status(P.status, DEV_RANGE);
-              origin[s] = make_int4(__float_as_int((float)sw0), __float_as_int((float)sh0), vb + l, snh);
-              vstage[s] = P.v[vb + l];
+              origin[s] = make_int4(__float_as_int((float)sw0), __float_as_int((float)sh0), vl, snh);
+              vstage[s] = P.v[vl];
               dev::mbar_arrive_expect_tx(&full[s], bytes);
-              dev::tma_load_3d(smem_raw + (size_t)s * stage_bytes, &tmap, &full[s], sw0, sh0,
-                               P.view0 + vb + l);
+              dev::tma_load_3d(smem_raw + (size_t)s * stage_bytes, &tmap, &full[s], sw0, sh0, P.view0 + vl);
             }
           }
           if (!__shfl_sync(0xffffffffu, ok, 0)) {
@@ -931,14 +931,12 @@ __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_c
   int tx, ty, tz;
   const uint32_t rank = SPLIT ? cluster_rank() : 0, nrank = SPLIT ? cluster_size() : 1;
   fdk_tile(P, P.tile0 + (SPLIT ? blockIdx.x / nrank : blockIdx.x), tx, ty, tz);
-  // this CTA's views, in batches of 32: a run of them, or (PI window, where few reach the tile)
-  // every nrank-th batch
-  int v0 = 0, v1 = P.nviews, vstep = 32;
+  // this CTA's views, tested 32 at a time: a run of them, or (PI window, where those that reach the
+  // tile follow each other) every nrank-th view
+  int v0 = 0, v1 = P.nviews;
+  const int vstep = SPLIT && PIW ? (int)nrank : 1;
   if constexpr (SPLIT && !PIW) split_views(P.nviews, rank, nrank, &v0, &v1);
-  if constexpr (SPLIT && PIW) {
-    v0 = 32 * (int)rank;
-    vstep = 32 * (int)nrank;
-  }
+  if constexpr (SPLIT && PIW) v0 = (int)rank;
 
   if (threadIdx.x == 0) {
     for (int k = 0; k < S; k++) dev::mbar_init(&full[k], 1);
@@ -955,7 +953,7 @@ __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_c
     if (lane == 0) dev::tma_prefetch(&tmap);
     const uint32_t bytes = (uint32_t)(stage_elems * 2);
     // views in order, 32 tested at a time (PI window: those that reach the tile)
-    int vb = v0 - vstep;
+    int vb = v0 - 32 * vstep;
     unsigned msk = 0;
     int lw0 = 0, lh0 = 0, lnw = 0, lnh = 0;
     bool exhausted = false, stalled = false, failed = false;
@@ -968,12 +966,12 @@ __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_c
         return;
       }
       while (msk == 0) {
-        vb += vstep;
+        vb += 32 * vstep;
         if (vb >= v1) {
           exhausted = true;
           return;
         }
-        const int v = vb + lane;
+        const int v = vb + lane * vstep;
         bool need = false;
         if (v < v1) {
           float fp[4];
@@ -982,16 +980,16 @@ __global__ void __launch_bounds__(FDK_THREADS, 3) fdk_pair_kernel(const __grid_c
         }
         msk = __ballot_sync(0xffffffffu, need);
       }
-      const int l = __ffs(msk) - 1;
+      const int l = __ffs(msk) - 1, vl = vb + l * vstep;
       msk &= msk - 1;
       const int w0 = __shfl_sync(0xffffffffu, lw0, l), h0 = __shfl_sync(0xffffffffu, lh0, l);
       const int nw = __shfl_sync(0xffffffffu, lnw, l), nh = __shfl_sync(0xffffffffu, lnh, l);
       const int s = is;  // free: its previous view has been rewritten
       if (lane == 0) {
         if (nw > P.BW || nh > P.BH) dev::record_status(P.status, DEV_RANGE);
-        sorg[s] = make_int4(__float_as_int((float)w0), __float_as_int((float)h0), vb + l, nh);
+        sorg[s] = make_int4(__float_as_int((float)w0), __float_as_int((float)h0), vl, nh);
         dev::mbar_arrive_expect_tx(&full[s], bytes);
-        dev::tma_load_3d(smem_raw + (size_t)s * stage_bytes, &tmap, &full[s], w0, h0, P.view0 + vb + l);
+        dev::tma_load_3d(smem_raw + (size_t)s * stage_bytes, &tmap, &full[s], w0, h0, P.view0 + vl);
       }
       __syncwarp();
       issued++;
@@ -1442,6 +1440,7 @@ struct fcb_bp_plan {
   int ptype = FCB_F32;
   int path = 0;  // 0 generic, 1 tma
   int device = 0;
+  int sms = 148;
   int nz_tile = 32;
   int maxv = FDK_MAXV;
   int BW = 0, BH = 0, stages = 0, pbufs = 0, wshift = 2;
@@ -1478,18 +1477,60 @@ size_t fdk_pair_smem_bytes(int BW, int BH, int stages, int pbufs, size_t record 
          (size_t)pbufs * record + (size_t)(stages + 2 * pbufs) * sizeof(uint64_t);
 }
 
-// Ranks that share a tile's views (1: none) for `ntiles` tiles and `nviews` views.  The chip holds
-// 444 CTAs, three per SM.  Clusters of six fill the SMs of a GPC best; below 40 tiles eight ranks
-// reach more SMs, up to 800 tiles two shorten the second wave, beyond that a tile alone is faster.
-// One B200, 180 views, FP32, milliseconds with 1, 2, 4, 6 and 8 ranks: 32 tiles (64^3) 0.191, 0.107,
-// 0.058, 0.058, 0.046; 108 tiles (96^3) 0.194, 0.155, 0.147, 0.124, 0.132; 256 tiles (128^3) 0.283,
-// 0.281, 0.275, 0.249, 0.283 (BF16 0.326, 0.313, 0.302, 0.273, 0.308); 500 tiles (160^3) 0.524,
-// 0.465, 0.492, 0.481, 0.530; 864 tiles (192^3) 0.766, 0.775, 0.807, 0.799, 0.898.
-int split_ranks(int ntiles, int nviews)
+// Ranks that share a tile's views (1: none) for a launch of `ntiles` tiles and `nviews` views, of which
+// an SM holds `resident` CTAs (3 unless the staged boxes are large).  A launch of S ranks per tile has
+// ceil(ntiles / room(S)) CTAs on the busiest SM, room(S) being the tiles that one CTA per SM takes
+// (clusters do not fill a GPC's SMs evenly), each with nviews / S views and what starting it and adding
+// its sums cost, about 1.2 views.  How long an SM takes for a view of each of its L CTAs, in units of one
+// CTA's, is `load` below.  Fitted to 720 launches on one B200 (1 to 780 tiles; 24 to 180 views; FP32,
+// BF16 and repacked rows; boxes of 44 x 50 to 124 x 184), every S from 1 to 8 timed: the choice costs
+// 1.1 % on average against the best, 4 % at most against one rank.  180 views, FP32, one rank against the
+// choice: 32 tiles 0.203 -> 0.060 ms (8), 108 tiles 0.207 -> 0.136 (6), 256 tiles 0.294 -> 0.261 (6), 500
+// tiles 0.541 -> 0.478 (2), 726 tiles 0.658 (1; 2 ranks 0.668).
+// PI window (`hits`: about as many of the launch's views reach a tile, half a turn of them): not the same
+// number each, so that more ranks even the tiles out.  Measured by itself (32 to 980 tiles, 160 to 4000
+// views, FP32 and BF16): 72 tiles, 600 views 0.312 -> 0.141 ms (6), 400 tiles 0.435 -> 0.351 (6), 720
+// tiles, 2000 views 2.59 -> 1.86 (2), 240 views 0.223 (1; 2 ranks 0.226).
+int split_ranks(int sms, int ntiles, int nviews, size_t smem, bool b16, bool piw = false, double hits = 0.0)
 {
   if (const char* e = getenv("FCB_FDK_SPLIT")) return std::max(1, std::min(8, atoi(e)));  // tuning knob
-  const int s = ntiles >= 800 ? 1 : ntiles > 444 ? 2 : ntiles >= 40 ? 6 : 8;
-  return std::max(1, std::min(s, nviews / 8));
+  const int resident = std::max(1, std::min(3, (int)((228 * 1024) / (smem + 1024))));
+  const double tiles = ntiles * (148.0 / sms);
+  double views = nviews;
+  if (piw) {
+    if (resident == 3) {
+      const int s = tiles >= 800 || (tiles > 600 && hits < 80) ? 1 : tiles > 444 ? 2 : tiles >= 40 ? 6 : 8;
+      return std::max(1, std::min(s, nviews / 8));
+    }
+    views = hits;
+  }
+  auto load = [&](double l) {
+    if (l <= 1.0) return 1.0;
+    if (resident == 1) return l;
+    if (resident == 2) return floor(0.5 * l) * (b16 ? 1.27 : 1.85) + fmod(l, 2.0);
+    return b16 ? 0.3 + 0.7 * l : 0.1 + 0.68 * l;
+  };
+  static const int ranks[4] = {2, 4, 6, 8};
+  static const double room[3][4] = {{73, 32, 20.5, 13}, {74, 33, 22, 15}, {74, 34, 23.4, 16.3}};
+  int best = 1;
+  double cost = views * load(ceil(tiles / 148.0)) * (resident == 3 ? 0.97 : 0.93);
+  for (int k = 0; k < 4; k++) {
+    // (eight fit a GPC's SMs worst: 75 tiles, 60 views 60.7 us, with six 56.7)
+    if (ranks[k] * 3 > views || (ranks[k] == 8 && tiles > 50)) break;
+    const double c = (views / ranks[k] + 1.2) * load(ceil(tiles / room[resident - 1][k] - 1e-9));
+    if (c < cost) {
+      cost = c;
+      best = ranks[k];
+    }
+  }
+  return best;
+}
+
+// Views of a PI-window launch that reach a tile, about: those of half a turn.
+double window_hits(const Problem& pb, const FdkParams& P)
+{
+  const double span = fabs(pb.angle[P.view0 + P.nviews - 1] - pb.angle[P.view0]);
+  return span > M_PI ? P.nviews * (M_PI / span) : P.nviews;
 }
 
 // One launch of a staged kernel: `split` ranks per tile in clusters of that many CTAs.
@@ -1510,7 +1551,9 @@ int launch_staged(Kern kern, size_t smem, int ntiles, int split, const CUtensorM
   at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
   cfg.numAttrs = split > 1 ? 1 : 0;
-  FCB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, map, P));
+  // (by address: the templated form copies the 29 KB of parameters once more)
+  void* args[] = {const_cast<CUtensorMap*>(&map), const_cast<FdkParams*>(&P)};
+  FCB_CUDA_TRY(cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kern), args));
   return FCB_OK;
 }
 
@@ -1526,11 +1569,10 @@ int launch_fdk(fcb_bp_plan* pl, const CUtensorMap& map, int chunk, int tz0, int 
     const int ntiles = (tz1 - tz0) * layer;
     if (ntiles <= 0) continue;
     if constexpr (X2 && NZ == 32 && MINB == fdk_min_blocks<NZ>()) {
-      const int split = split_ranks(ntiles, P.nviews);
+      const size_t smem = fdk_smem_bytes(pl->BW, pl->BH, pl->stages, sizeof(T), sizeof(FdkView), true);
+      const int split = split_ranks(pl->sms, ntiles, P.nviews, smem, false, PIW, PIW ? window_hits(pl->pb, P) : 0.0);
       if (split > 1) {
-        FCB_TRY(launch_staged(fdk_tma_kernel<T, NZ, PIW, X2, MINB, false, true>,
-                              fdk_smem_bytes(pl->BW, pl->BH, pl->stages, sizeof(T), sizeof(FdkView), true), ntiles,
-                              split, map, P, st));
+        FCB_TRY(launch_staged(fdk_tma_kernel<T, NZ, PIW, X2, MINB, false, true>, smem, ntiles, split, map, P, st));
         continue;
       }
     }
@@ -1551,8 +1593,10 @@ int launch_fdk_pair(fcb_bp_plan* pl, const CUtensorMap& map, int chunk, int tz0,
     P.tile0 = tz0 * layer;
     const int ntiles = (tz1 - tz0) * layer;
     if (ntiles <= 0) continue;
-    const int split = split_ranks(ntiles, P.nviews);
-    const size_t smem = fdk_pair_smem_bytes(pl->BW, pl->BH, pl->stages, pl->pbufs, sizeof(FdkView), split > 1);
+    const size_t need = fdk_pair_smem_bytes(pl->BW, pl->BH, pl->stages, pl->pbufs, sizeof(FdkView), true);
+    const int split = split_ranks(pl->sms, ntiles, P.nviews, need, true, PIW, PIW ? window_hits(pl->pb, P) : 0.0);
+    const size_t smem =
+        split > 1 ? need : fdk_pair_smem_bytes(pl->BW, pl->BH, pl->stages, pl->pbufs, sizeof(FdkView), false);
     if (split > 1)
       FCB_TRY(launch_staged(fdk_pair_kernel<T, 32, PIW, false, true>, smem, ntiles, split, map, P,
                             st));
@@ -1566,15 +1610,19 @@ int launch_fdk_pair(fcb_bp_plan* pl, const CUtensorMap& map, int chunk, int tz0,
 template <typename T>
 int launch_matrix(const fcb_bp_plan* pl, const CUtensorMap& map, const FdkParams& P, int ntiles, cudaStream_t st)
 {
-  const int split = split_ranks(ntiles, P.nviews);
   if constexpr (sizeof(T) == 4) {
-    const size_t smem = fdk_smem_bytes(pl->BW, pl->BH, pl->stages, sizeof(T), sizeof(GenView), split > 1);
+    const size_t need = fdk_smem_bytes(pl->BW, pl->BH, pl->stages, sizeof(T), sizeof(GenView), true);
+    const int split = split_ranks(pl->sms, ntiles, P.nviews, need, false);
+    const size_t smem = split > 1 ? need : fdk_smem_bytes(pl->BW, pl->BH, pl->stages, sizeof(T), sizeof(GenView), false);
     if (split > 1)
       return launch_staged(fdk_tma_kernel<float, 32, false, true, 3, true, true>, smem, ntiles,
                            split, map, P, st);
     return launch_staged(fdk_tma_kernel<float, 32, false, true, 3, true>, smem, ntiles, 1, map, P, st);
   } else {
-    const size_t smem = fdk_pair_smem_bytes(pl->BW, pl->BH, pl->stages, pl->pbufs, sizeof(GenView), split > 1);
+    const size_t need = fdk_pair_smem_bytes(pl->BW, pl->BH, pl->stages, pl->pbufs, sizeof(GenView), true);
+    const int split = split_ranks(pl->sms, ntiles, P.nviews, need, true);
+    const size_t smem =
+        split > 1 ? need : fdk_pair_smem_bytes(pl->BW, pl->BH, pl->stages, pl->pbufs, sizeof(GenView), false);
     if (split > 1)
       return launch_staged(fdk_pair_kernel<T, 32, false, true, true>, smem, ntiles, split, map, P,
                            st);
@@ -1712,6 +1760,10 @@ static int bp_plan_build(const fcb_geometry* g, int kernelMode, int projType, in
   pl->mode = kernelMode == 0 ? 0 : (kernelMode == 1 ? 1 : 2);
   pl->ptype = projType;
   cudaGetDevice(&pl->device);
+  if (cudaDeviceGetAttribute(&pl->sms, cudaDevAttrMultiProcessorCount, pl->device) != cudaSuccess) {
+    cudaGetLastError();
+    pl->sms = 148;
+  }
   const int nx = pb.volEnd[0] - pb.volStart[0], ny = pb.volEnd[1] - pb.volStart[1],
             nz = pb.volEnd[2] - pb.volStart[2];
   pl->updates = (long long)nx * ny * nz * pb.nviews;
