@@ -1477,6 +1477,36 @@ size_t fdk_pair_smem_bytes(int BW, int BH, int stages, int pbufs, size_t record 
          (size_t)pbufs * record + (size_t)(stages + 2 * pbufs) * sizeof(uint64_t);
 }
 
+// CTAs that an SM holds at `smem` bytes of dynamic shared memory each (registers allow three).
+int resident_ctas(size_t smem) { return std::max(1, std::min(3, (int)((228 * 1024) / (smem + 1024)))); }
+
+// Words added to the rows of an FP32 box of BW x BH.  The lanes of a warp (8 x 4 columns) read a dozen
+// columns of a few neighbouring rows: at 12 or 20 mod 32 words those spread over the banks, at 16 every
+// second row meets, near a multiple of 32 all do; and a wider box may cost a CTA per SM.  Time
+// against the best of eight pitches by the distance from a multiple of 32, and by CTAs per SM, measured on
+// 130 geometries (boxes of 24 x 29 to 136 x 211, one B200): the choice costs 0.3 % on average, the width
+// as it comes 12 %, 4 mod 8 words 6 %.  256^3 / 90 views at pitch 1.0 (44 against 36 words) 0.876 ms
+// against 0.953, at 0.6 (76 against 56) 0.993 against 1.34; 128^3 / 180 views at 0.5 (76 against 60) 0.314
+// against 0.404; 256 x 256 x 512 / 60 views at 0.9 (52 against 48) 1.37 against 1.70.
+int box_pad(int BW, int BH)
+{
+  static const double three[5] = {1.5, 1.2, 1.06, 1.0, 1.08}, one[5] = {1.12, 1.05, 1.02, 1.0, 1.01};
+  static const double share[4] = {0.0, 1.65, 1.1, 1.0};
+  int best = 0;
+  double cost = 0.0;
+  for (int pad = 0; pad <= 20; pad += 4) {
+    const size_t smem = fdk_smem_bytes(BW + pad, BH, 2, 4);
+    if (BW + pad > 256 || smem > 227 * 1024) break;
+    const int n = resident_ctas(smem), d = std::min((BW + pad) % 32, 32 - (BW + pad) % 32) / 4;
+    const double c = (n > 1 ? three : one)[d] * share[n] * (1.0 + 0.001 * pad);
+    if (pad == 0 || c < cost) {
+      cost = c;
+      best = pad;
+    }
+  }
+  return best;
+}
+
 // Ranks that share a tile's views (1: none) for a launch of `ntiles` tiles and `nviews` views, of which
 // an SM holds `resident` CTAs (3 unless the staged boxes are large).  A launch of S ranks per tile has
 // ceil(ntiles / room(S)) CTAs on the busiest SM, room(S) being the tiles that one CTA per SM takes
@@ -1494,7 +1524,7 @@ size_t fdk_pair_smem_bytes(int BW, int BH, int stages, int pbufs, size_t record 
 int split_ranks(int sms, int ntiles, int nviews, size_t smem, bool b16, bool piw = false, double hits = 0.0)
 {
   if (const char* e = getenv("FCB_FDK_SPLIT")) return std::max(1, std::min(8, atoi(e)));  // tuning knob
-  const int resident = std::max(1, std::min(3, (int)((228 * 1024) / (smem + 1024))));
+  const int resident = resident_ctas(smem);
   const double tiles = ntiles * (148.0 / sms);
   double views = nviews;
   if (piw) {
@@ -1884,20 +1914,9 @@ static int bp_plan_build(const fcb_geometry* g, int kernelMode, int projType, in
     pl->BH = h[1] + 1;  // + 1: the inner z layers' corner floors (see fdk_footprint_kernel)
     if (pl->BW < align) pl->BW = align;
     if (pl->BH < 2) pl->BH = 2;
-    // FP32 boxes: the row pitch decides the bank conflicts, since the lanes of a warp (8 x 4
-    // columns) read a dozen columns of a few neighbouring rows.  At 12 to 20 mod 32 words those
-    // spread over the banks for every detector pitch from 0.5 to 1.6 voxels (1.0 to 1.25 wavefronts
-    // per load); next to a multiple of 32 they collide (1.2 to 2).  One B200, padded against the
-    // width as it comes: 256^3 / 90 views at pitch 1.0 (44 against 36 words) 0.876 ms against
-    // 0.953, at 0.6 (76 against 56) 0.993 against 1.34; 128^3 / 180 views at 0.5 (76 against 60)
-    // 0.314 ms against 0.404.  PI-window launches, bound by their window tests, keep the smaller
-    // box (helix: 56.2 ms at 36 words, 56.4 at 44), at 4 mod 8 words.
-    if (projType == FCB_F32 && piwin) {
-      if (pl->BW % 8 == 0) pl->BW += 4;
-    } else if (projType == FCB_F32) {
-      const int r = pl->BW % 32, pad = r < 12 ? 12 - r : r > 20 ? 44 - r : 0;
-      if (pl->BW + pad <= 256 && fdk_smem_bytes(pl->BW + pad, pl->BH, 2, 4) <= 100 * 1024) pl->BW += pad;
-    }
+    // FP32 boxes: see box_pad.  PI-window launches, bound by their window tests, keep the smaller box
+    // (helix: 56.2 ms at 36 words, 56.4 at 44), at 4 mod 8 words.
+    if (projType == FCB_F32) pl->BW += !piwin ? box_pad(pl->BW, pl->BH) : pl->BW % 8 == 0 ? 4 : 0;
     // the largest dynamic shared memory a CTA of this device may opt into
     int smem_optin = 227 * 1024;  // sm_100
     if (cudaDeviceGetAttribute(&smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, pl->device) !=
