@@ -1511,10 +1511,10 @@ int box_pad(int BW, int BH)
 // an SM holds `resident` CTAs (3 unless the staged boxes are large).  A launch of S ranks per tile has
 // ceil(ntiles / room(S)) CTAs on the busiest SM, room(S) being the tiles that one CTA per SM takes
 // (clusters do not fill a GPC's SMs evenly), each with nviews / S views and what starting it and adding
-// its sums cost, about 1.2 views.  How long an SM takes for a view of each of its L CTAs, in units of one
-// CTA's, is `load` below.  Fitted to 720 launches on one B200 (1 to 780 tiles; 24 to 180 views; FP32,
+// its sums cost: about 1.2 views among three CTAs, 3 and 4 among two and one, where less of it hides behind
+// the others.  How long an SM takes for a view of each of its L CTAs, in units of one CTA's, is `load` below.  Fitted to 720 launches on one B200 (1 to 780 tiles; 24 to 180 views; FP32,
 // BF16 and repacked rows; boxes of 44 x 50 to 124 x 184), every S from 1 to 8 timed: the choice costs
-// 1.1 % on average against the best, 4 % at most against one rank.  180 views, FP32, one rank against the
+// 1 % on average against the best, nothing against one rank.  180 views, FP32, one rank against the
 // choice: 32 tiles 0.203 -> 0.060 ms (8), 108 tiles 0.207 -> 0.136 (6), 256 tiles 0.294 -> 0.261 (6), 500
 // tiles 0.541 -> 0.478 (2), 726 tiles 0.658 (1; 2 ranks 0.668).
 // PI window (`hits`: about as many of the launch's views reach a tile, half a turn of them): not the same
@@ -1541,13 +1541,14 @@ int split_ranks(int sms, int ntiles, int nviews, size_t smem, bool b16, bool piw
     return b16 ? 0.3 + 0.7 * l : 0.1 + 0.68 * l;
   };
   static const int ranks[4] = {2, 4, 6, 8};
+  static const double start[3] = {4.0, 3.0, 1.2};
   static const double room[3][4] = {{73, 32, 20.5, 13}, {74, 33, 22, 15}, {74, 34, 23.4, 16.3}};
   int best = 1;
   double cost = views * load(ceil(tiles / 148.0)) * (resident == 3 ? 0.97 : 0.93);
   for (int k = 0; k < 4; k++) {
     // (eight fit a GPC's SMs worst: 75 tiles, 60 views 60.7 us, with six 56.7)
     if (ranks[k] * 3 > views || (ranks[k] == 8 && tiles > 50)) break;
-    const double c = (views / ranks[k] + 1.2) * load(ceil(tiles / room[resident - 1][k] - 1e-9));
+    const double c = (views / ranks[k] + start[resident - 1]) * load(ceil(tiles / room[resident - 1][k] - 1e-9));
     if (c < cost) {
       cost = c;
       best = ranks[k];
