@@ -960,7 +960,7 @@ __global__ void __launch_bounds__(WGT_THREADS, 1) conv3d16_wgrad_tc_kernel(const
     // ---------------------------------------------------------------- MMA issuer
     if (lane == 0) {
       const uint32_t xbase = dev::smem_u32(X);
-      // M = 128 (rows 0-47 used), N = 48, A K-major in TMEM, B MN-major in shared memory
+      // M = 128 (rows 0-47 used), N = 144, A K-major in TMEM, B MN-major in shared memory
       constexpr uint32_t IDESC = tc::idesc_bf16(CV_TILE, 144) | (1u << 16);
       int i = 0, n = 0;
       bool failed = false;
@@ -976,7 +976,7 @@ __global__ void __launch_bounds__(WGT_THREADS, 1) conv3d16_wgrad_tc_kernel(const
             break;
           }
           tc::fence_after();
-          // MN-major B over the slots of rows y-1, y, y+1 of one dz: N core matrices (dy, ci
+          // MN-major B over the slots of rows y-1, y, y+1, three planes each: N core matrices (dy, dz, ci
           // half) every WGT_RB bytes (SBO), K core matrices of 8 voxels every 128 bytes (LBO);
           // a K-step of 16 voxels moves the start address by 256 B (16 in the descriptor's
           // address field, which stays below 2^14 inside shared memory)
@@ -993,7 +993,7 @@ __global__ void __launch_bounds__(WGT_THREADS, 1) conv3d16_wgrad_tc_kernel(const
       else dev::mbar_arrive(fin);
     }
   } else if ((warp & 3) < 2) {
-    // ---------------------------------------------------------------- A writers (warps 0-1, 4-5, ..)
+    // ---------------------------------------------------------------- A writers (warps 0-1 and 4-5)
     const int group = warp >> 2;
     const int s0 = 2 * (warp & 1);  // first of the shifts s = 0, 1 or s = 2 (TMEM lanes 16 s + co)
     const uint32_t lane_base = (uint32_t)(16 * s0) << 16;
@@ -1176,7 +1176,8 @@ static_assert(CGP_BLOCKS * 8 == FCB_CONV_GRAD_SCRATCH, "gradient scratch");
 // box row at a time, and rows of 16 bytes fetch every sector twice.  A tile's box starts one group
 // before its first voxel, its operands 2^gs - 1 voxels into the box, so gs <= `most` must divide nx.
 // The weight gradient takes groups of up to 8 (256^3: 0.468 ms, with pairs 0.49); the forward
-// kernel, not bound by its copies, pairs (groups of 8: 0.444 ms, with pairs 0.440).
+// kernel, not bound by its copies, pairs, whose margins fit its stages (groups of 8 made no difference
+// to the kernel before it, which staged three rows of one plane: 0.444 ms against 0.440).
 static int box_group(int nx, int most)
 {
   int gs = most;
@@ -1194,7 +1195,7 @@ try {
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   CUtensorMap map;
   // FCB_CONV_SIMPLE=1: one CTA per tile; FCB_CONV_SIMPLE=2: persistent without row reuse (both for
-  // comparison, one channel half of one row per box); default: three dy taps per MMA
+  // comparison, one channel half of one row per box); default: three dz taps per MMA
   const char* env = getenv("FCB_CONV_SIMPLE");
   const int variant = env ? atoi(env) : 0;
   const bool simple = variant == 1 || variant == 2;

@@ -12,7 +12,8 @@
 //      and length correction g2 = D / sqrt(u^2+D^2+v^2) g1
 //   2. forward height rebinning onto kappa-lines v_k(u, psi) = P/(2 pi)(psi + psi/tan(psi) u/D)
 //      (per-(kappa, column) interpolation table built on the host in FP64); both stages are
-//      kats_kappa_kernel, which keeps g2 in shared memory
+//      kats_kappa_kernel, which keeps g2 in shared memory, above 768 rows (and for less than 16
+//      above rf::RC_MAX_W columns) kats_deriv_kernel and kats_rebin_fwd_kernel
 //   3. Hilbert transform along u, band-limited kernel (1 - cos(pi n))/(pi n): a linear
 //      convolution, in place by the one-pass row transform (fcb_rowfft.cuh), for rows above
 //      rf::RC_MAX_W by cuFFT on zero-padded rows; kats_hilbert_kernel is the direct O(W^2) form,
@@ -119,38 +120,43 @@ __device__ __forceinline__ float kats_deriv(const KatsColumn& X, int j, int H, i
   return g1 * (K.D * rsqrtf(X.q2 + v * v));
 }
 
-// Derivative and forward rebinning: the kappa rows of views t0 + blockIdx.y * KK_VIEWS ... (nv of
+// What a column of view `tl` of the batch from view t0 on differentiates; `before` is view
+// t0 - 1 (null at the first view).
+__device__ __forceinline__ KatsColumn kats_view(const float* g, const float* before, int t0, int tl, int n, size_t plane,
+                                                int i, int W, const KatsDerivConst& C)
+{
+  const int t = t0 + tl;
+  const float* c = g + (size_t)t * plane;
+  return kats_column(t == 0 ? nullptr : tl == 0 ? before : c - plane, c, t + 1 < n ? c + plane : nullptr, i, W, C);
+}
+
+// Derivative and forward rebinning: the kappa rows of views t0 + blockIdx.y * kv ... (nv of
 // them in all), columns blockIdx.x * 32 + lane, at a row pitch of L:
 //   out[tl][k][i] = g2[j0] * (1 - a) + g2[j0 + 1] * a from the (kappa, column) table (j0, a).
-// The strip's derivatives of one view sit in shared memory between the two (STAGE), since each is
-// read about 2 K / H times (the strip takes 128 bytes a row: up to 768 rows leave two CTAs per SM);
-// beyond that every tap is derived where it is read.
-// `before` is view t0 - 1 (null at the first view).  I: as in kats_deriv, for the K L values too.
+// The strip's derivatives of one view sit in shared memory between the two, since each is read about
+// 2 K / H times (the strip takes 128 bytes a row: up to 768 rows leave two CTAs per SM).  A CTA takes
+// KK_VIEWS views where that leaves 20 CTAs' views per SM (736 x 64, 4640 views: 3.50 ms for the whole
+// filter, 3.58 with one), else one (64 x 700, 80 views: 80 us, 178 with four).
+// I: as in kats_deriv, for the K L values too.
 constexpr int KK_VIEWS = 4;
-template <bool STAGE, typename I>
+template <typename I>
 __global__ void __launch_bounds__(256, 5) kats_kappa_kernel(const float* __restrict__ g,
                                                             const float* __restrict__ before,
                                                             float* __restrict__ out, const float2* __restrict__ tab,
-                                                            int n, int H, int W, int K, int L, int t0, int nv,
+                                                            int n, int H, int W, int K, int L, int t0, int nv, int kv,
                                                             const KatsDerivConst C)
 {
   extern __shared__ float kk_g2[];  // [H][32]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int i = blockIdx.x * 32 + lane;
-  const size_t plane = (size_t)H * W;
-  const int l0 = blockIdx.y * KK_VIEWS, l1 = min(nv, l0 + KK_VIEWS);
+  const int l0 = blockIdx.y * kv, l1 = min(nv, l0 + kv);
   for (int tl = l0; tl < l1; tl++) {
-    const int t = t0 + tl;
-    const float* c = g + (size_t)t * plane;
-    const KatsColumn X =
-        kats_column(t == 0 ? nullptr : tl == 0 ? before : c - plane, c, t + 1 < n ? c + plane : nullptr, i, W, C);
-    if constexpr (STAGE) {
-      if (i < W) {
+    if (i < W) {
+      const KatsColumn X = kats_view(g, before, t0, tl, n, (size_t)H * W, i, W, C);
 #pragma unroll 2
-        for (int j = warp; j < H; j += 8) kk_g2[j * 32 + lane] = kats_deriv<I>(X, j, H, W, C);
-      }
-      __syncthreads();
+      for (int j = warp; j < H; j += 8) kk_g2[j * 32 + lane] = kats_deriv<I>(X, j, H, W, C);
     }
+    __syncthreads();
     if (i < W) {
       float* row = out + (size_t)tl * K * L;
 #pragma unroll 4
@@ -159,14 +165,54 @@ __global__ void __launch_bounds__(256, 5) kats_kappa_kernel(const float* __restr
         const int j0 = __float_as_int(ja.x);
         float val = 0.0f;
         if (j0 >= 0) {  // (and at most H - 2)
-          const float v0 = STAGE ? kk_g2[j0 * 32 + lane] : kats_deriv<I>(X, j0, H, W, C);
-          const float v1 = STAGE ? kk_g2[j0 * 32 + lane + 32] : kats_deriv<I>(X, j0 + 1, H, W, C);
+          const float v0 = kk_g2[j0 * 32 + lane], v1 = kk_g2[j0 * 32 + lane + 32];
           val = fmaf(ja.y, v1 - v0, v0);
         }
         row[(I)k * (I)L + (I)i] = val;
       }
     }
-    if constexpr (STAGE) __syncthreads();
+    __syncthreads();
+  }
+}
+
+// The same in two passes over global memory, columns across the CTA and KK_ROWS rows or lines per CTA
+// (blockIdx.z), for detectors too tall to stage a strip (128 x 1000, 80 views: 176 us for the whole
+// filter, 511 where every tap was derived where it is read), and for a few rows beyond the row transform's
+// length, whose strips are too little work per CTA (8192 x 8, 600 views: 1.41 ms, 1.51 staged).
+constexpr int KK_ROWS = 16;
+template <typename I>
+__global__ void __launch_bounds__(256) kats_deriv_kernel(const float* __restrict__ g, const float* __restrict__ before,
+                                                         float* __restrict__ g2, int n, int H, int W, int t0,
+                                                         const KatsDerivConst C)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, tl = blockIdx.y;
+  if (i >= W) return;
+  const KatsColumn X = kats_view(g, before, t0, tl, n, (size_t)H * W, i, W, C);
+  float* out = g2 + (size_t)tl * H * W;
+  const int j0 = blockIdx.z * KK_ROWS, j1 = min(H, j0 + KK_ROWS);
+#pragma unroll 4
+  for (int j = j0; j < j1; j++) out[(I)j * (I)W + (I)i] = kats_deriv<I>(X, j, H, W, C);
+}
+template <typename I>
+__global__ void __launch_bounds__(256) kats_rebin_fwd_kernel(const float* __restrict__ g2, float* __restrict__ out,
+                                                             const float2* __restrict__ tab, int H, int W, int K, int L)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, tl = blockIdx.y;
+  if (i >= W) return;
+  const float* col = g2 + (size_t)tl * H * W + i;
+  float* row = out + (size_t)tl * K * L;
+  const int k0 = blockIdx.z * KK_ROWS, k1 = min(K, k0 + KK_ROWS);
+#pragma unroll 4
+  for (int k = k0; k < k1; k++) {
+    const float2 ja = __ldg(tab + ((I)k * (I)W + (I)i));
+    const int j0 = __float_as_int(ja.x);
+    float val = 0.0f;
+    if (j0 >= 0) {  // (and at most H - 2)
+      const float* c = col + (I)j0 * (I)W;
+      const float v0 = c[0], v1 = c[W];
+      val = fmaf(ja.y, v1 - v0, v0);
+    }
+    row[(I)k * (I)L + (I)i] = val;
   }
 }
 
@@ -265,6 +311,10 @@ static double frac_index(const std::vector<double>& xs, double x)
   return lo + (x - xs[lo]) / (xs[hi] - xs[lo]);
 }
 
+// A strip of 32 columns of a view's derivatives, and whether it is staged (see kats_kappa_kernel).
+static size_t kats_strip(int H) { return (size_t)H * 32 * sizeof(float); }
+static bool kats_staged(int H, int W) { return kats_strip(H) <= 96 * 1024 && (W <= rf::RC_MAX_W || H >= 16); }
+
 static float int_bits(int v)
 {
   float f;
@@ -285,6 +335,8 @@ struct fcb_katsevich_plan {
   float* dba = nullptr;
   float* g4 = nullptr;     // kappa rows of one batch [vb][K][L], transformed in place
   float* edge = nullptr;   // the view before a batch, when out is in
+  float* g2 = nullptr;     // two passes: derivatives of one batch [vb][H][W]
+  int sms = 148;
   rf::RowConv conv;  // rows up to rf::RC_MAX_W
   // longer rows: cuFFT
   int nb = 0;
@@ -296,7 +348,7 @@ struct fcb_katsevich_plan {
   {
     if (pf) cufftDestroy(pf);
     if (pi) cufftDestroy(pi);
-    cudaFree(g3); cudaFree(g4); cudaFree(edge); cudaFree(dfja); cudaFree(dba); cudaFree(dbk);
+    cudaFree(g3); cudaFree(g4); cudaFree(g2); cudaFree(edge); cudaFree(dfja); cudaFree(dba); cudaFree(dbk);
     cudaFree(hspec); cudaFree(dhim);
   }
 };
@@ -358,6 +410,8 @@ try {
   auto* pl = new fcb_katsevich_plan();
   pl->nviews = nviews; pl->H = H; pl->W = W; pl->K = K;
   pl->dlam = (float)dlam; pl->pw = pw; pl->D = D; pl->su = (float)su;
+  int dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&pl->sms, cudaDevAttrMultiProcessorCount, dev);
   const bool fused = W <= rf::RC_MAX_W;
   int rc = FCB_OK;
   do {
@@ -383,7 +437,7 @@ try {
       // 4.10 ms, 128 MB 3.92, 256 MB 3.68, 512 MB 3.54, 1 GB 3.44).
       long long budget = 512ll << 20;
       if (const char* e = getenv("FCB_KATS_BATCH_MB")) budget = (long long)std::max(1, atoi(e)) << 20;
-      long long vb = std::max<long long>(1, budget / (4ll * pl->L * K));
+      long long vb = std::max<long long>(1, budget / (4ll * pl->L * (kats_staged(H, W) ? K : std::max(K, H))));
       const long long wave = pl->conv.wave_rows();
       if (vb * K >= wave) vb = vb * K / wave * wave / K;
       pl->vb = (int)std::min<long long>(nviews, std::max<long long>(1, vb));
@@ -394,7 +448,8 @@ try {
       pl->vb = (int)std::min<long long>(nviews, std::max<long long>(1, (256ll << 20) / (8ll * pl->nb * K)));
     }
     const long long rows = (long long)pl->vb * K;
-    if (cudaMalloc(&pl->edge, (size_t)H * W * 4) || cudaMalloc(&pl->g4, (size_t)rows * pl->L * 4)) {
+    if (cudaMalloc(&pl->edge, (size_t)H * W * 4) || cudaMalloc(&pl->g4, (size_t)rows * pl->L * 4) ||
+        (!kats_staged(H, W) && cudaMalloc(&pl->g2, (size_t)pl->vb * H * W * 4))) {
       cudaGetLastError();
       rc = set_error(FCB_ERR_NOMEM, "Katsevich filter scratch");
       break;
@@ -482,19 +537,26 @@ try {
       return set_error(FCB_ERR_CUDA, cudaGetErrorString(e));
     }
   }
-  const size_t strip = (size_t)H * 32 * sizeof(float);  // a view's derivatives in 32 columns
-  const bool stage = strip <= 96 * 1024;
-  const bool wide = std::max((long long)H * W, (long long)K * L) > 0x7fffffffll;
-  auto kappa = stage ? (wide ? kats_kappa_kernel<true, size_t> : kats_kappa_kernel<true, unsigned>)
-                     : (wide ? kats_kappa_kernel<false, size_t> : kats_kappa_kernel<false, unsigned>);
+  const bool stage = kats_staged(H, W);
+  const bool wide = std::max((long long)H * W, (long long)K * L) > 0x7fffffffll;  // 64-bit indices
+  auto kappa = wide ? kats_kappa_kernel<size_t> : kats_kappa_kernel<unsigned>;
+  auto deriv = wide ? kats_deriv_kernel<size_t> : kats_deriv_kernel<unsigned>;
+  auto rebin = wide ? kats_rebin_fwd_kernel<size_t> : kats_rebin_fwd_kernel<unsigned>;
   if (stage) FCB_CUDA_TRY(cudaFuncSetAttribute(kappa, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+  const unsigned strips = (unsigned)((W + 31) / 32), bx = std::min(256u, strips * 32), gx = (W + bx - 1) / bx;
   // one batch: kappa rows of views [t0, t0 + nv), their Hilbert transform, backward rebinning
   auto batch = [&](int t0, int nv) -> int {
     const long long rows = (long long)nv * K;
     float* g3 = fused || direct ? pl->g4 : pl->g3;
     const float* before = t0 == 0 ? nullptr : in == out ? pl->edge : src + (size_t)(t0 - 1) * plane;
-    const dim3 kg((W + 31) / 32, (nv + KK_VIEWS - 1) / KK_VIEWS);
-    kappa<<<kg, 256, stage ? strip : 0, st>>>(src, before, g3, pl->dfja, nviews, H, W, K, L, t0, nv, KC);
+    if (stage) {
+      const int kv = (long long)strips * nv >= 20ll * pl->sms ? KK_VIEWS : 1;
+      kappa<<<dim3(strips, (nv + kv - 1) / kv), 256, kats_strip(H), st>>>(src, before, g3, pl->dfja, nviews, H, W, K, L, t0,
+                                                                          nv, kv, KC);
+    } else {
+      deriv<<<dim3(gx, nv, (H + KK_ROWS - 1) / KK_ROWS), bx, 0, st>>>(src, before, pl->g2, nviews, H, W, t0, KC);
+      rebin<<<dim3(gx, nv, (K + KK_ROWS - 1) / KK_ROWS), bx, 0, st>>>(pl->g2, g3, pl->dfja, H, W, K, L);
+    }
     FCB_CUDA_TRY(cudaGetLastError());
     if (in == out && t0 + nv < nviews)
       FCB_CUDA_TRY(cudaMemcpyAsync(pl->edge, in + (size_t)(t0 + nv - 1) * plane, plane * sizeof(float),

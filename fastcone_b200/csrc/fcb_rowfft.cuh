@@ -31,7 +31,7 @@
 // widths from 32 to 2048, smooth rows, Ram-Lak with and without the weight and Shepp-Logan, 0.38
 // to 0.91 of cuFFT's.
 //
-// The stages are functions of (thread, row buffer) so that the host can run them too.
+// The stages are functions of (thread, row buffer), so that the host can run them too (a CPU test does).
 #pragma once
 
 #include <math.h>
@@ -524,9 +524,11 @@ __global__ void __launch_bounds__(K::T * K::GPC, 1) rowconv_kernel(const IO io, 
   }
 }
 
-// f(Config) for the smallest size N >= W (work grows with N; a width just above a size pays up
-// to a third more than its own, and still less than half of cuFFT's time at every width
-// measured from 48 to 4096); false when there is none (W > RC_MAX_W).
+// f(Config) for the smallest size N >= W (work grows with N: a width just above a size pays for the next
+// one and its fewer rows per SM, 64 x 256 rows of 512 and 513 values 63 and 89 us, 1024 and 1025 106 and
+// 182, 2048 and 2049 217 and 323, where cuFFT between its passes took 182 and 269, 345 and 1298, 682 and
+// 2731; at every width measured from 48 to 4096 less than half of its time); false when there is none
+// (W > RC_MAX_W).
 constexpr int RC_MAX_W = 4096;
 template <class F>
 bool rc_dispatch(int W, F&& f)

@@ -48,7 +48,9 @@ def backproject(proj: torch.Tensor, geom: ConeGeometry, mode: int = _lib.MODE_FD
 
 
 class BackprojectPlan:
-    """Geometry digested once; ``__call__`` queues the kernels and allocates nothing."""
+    """Geometry digested once; ``__call__`` queues the kernels and allocates nothing but stream-ordered
+    scratch for projections whose rows are not whole 16-byte groups (without it, and under capture,
+    such rows are read unstaged)."""
 
     def __init__(self, geom: ConeGeometry, mode: int = _lib.MODE_FDK, dtype=torch.float32):
         self.geom = geom
@@ -237,7 +239,8 @@ def katsevich_filter(proj: torch.Tensor, geom: ConeGeometry, n_kappa: int = 0,
 
 class KatsevichPlan:
     """Reusable Katsevich filter for geom's helix and detector (tables and
-    intermediate buffers made once); calls are stream-ordered and allocate nothing."""
+    intermediate buffers made once); calls are stream-ordered and allocate nothing (unless ``out``
+    overlaps the input without being it)."""
 
     def __init__(self, geom: ConeGeometry, n_kappa: int = 0):
         if geom.helical_pitch == 0.0:

@@ -239,8 +239,10 @@ int fcb_sync_status(void* stream);
 /* The host-buffer entry points (GPU_CB_*, fcb_backproject_host, fcb_project_host,
  * fcb_fbp_host) keep the device blocks of a finished call and reuse them in later calls
  * that fit (at most 8 blocks per device; a failed allocation first returns them), and
- * fcb_fbp_host keeps its filter plans (at most 4 per device).  This
- * returns everything kept to the driver.  FCB_HOST_CACHE=0 in the environment frees each
+ * fcb_fbp_host keeps its filter plans (at most 4 per device).  The device entry points that
+ * need scratch for the length of a call (one-shot projections, odd-row backprojections, filters whose
+ * buffers overlap) take it from a pool per device and context that keeps up to 1 GiB.  This
+ * returns everything kept (the pool of the caller's context) to the driver.  FCB_HOST_CACHE=0 in the environment frees each
  * call's blocks and plans when it ends instead. */
 int fcb_release_device_cache(void);
 
@@ -284,8 +286,9 @@ int fcb_katsevich_filter_device(const float* in, float* out, int nviews, int H, 
                                 void* stream);
 
 /* The same filter as a reusable plan for one helix and detector: kappa-line tables, the
- * Hilbert kernel's spectrum and the kappa rows of one batch of views made once (512 MiB at most; above
- * 4096 columns the Hilbert transform is cuFFT's, on 0.75 GiB batches); execute is stream-ordered, allocates nothing
+ * Hilbert kernel's spectrum and the kappa rows of one batch of views made once (512 MiB at most, unless
+ * one view takes more; above 768 rows as much again for their derivatives; above 4096 columns the
+ * Hilbert transform is cuFFT's, on 0.75 GiB batches); execute is stream-ordered, allocates nothing
  * (unless in and out overlap without being the same buffer: then a stream-ordered copy of in)
  * and does not synchronise.  One execute at a time per plan. */
 typedef struct fcb_katsevich_plan fcb_katsevich_plan;
